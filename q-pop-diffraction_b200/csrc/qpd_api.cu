@@ -17,6 +17,7 @@
 #include <cudaTypedefs.h>
 
 #include "qpopdiff.h"
+#include "qpd_any.h"
 #include "qpd_fast.cuh"
 #include "qpd_fields.cuh"
 #include "qpd_zpfa.cuh"
@@ -57,6 +58,7 @@ struct qpd_ctx {
     int nPhase = 0, nStruc = 0, precision = QPD_FP32, schedule = QPD_SCHED_FUSED;
     std::vector<int> radix[3];
     DevMem tw[3];
+    DevMem tw_any[3];  // the same in the order of the runtime-length passes (AnyStages)
 
     // crystal
     bool have_crystal = false;
@@ -77,6 +79,13 @@ struct qpd_ctx {
     // inside `tables` (have_p4y: ny = 4000, have_p4x: nx = 4000)
     bool have_p4y = false, have_p4x = false;
     qpd::Pass4k p4y, p4x;
+    // runtime-length passes: the stages of each axis (any_ok: its factors are covered) and the folds of the y and
+    // x passes and of the adjoint's x and y passes (n = 0: more inputs than one pass takes)
+    qpd::AnyStages any[3];
+    bool any_ok[3] = {false, false, false};
+    qpd::AnyFold anyY, anyX, anyAX, anyAY;
+    int sms = 0;
+    size_t smem_max = 0;
 
     // workspace
     DevMem fields;  // fused: 3 * ng1 fields; plain: buf + amp
@@ -639,6 +648,23 @@ template <typename T> struct Impl {
         for (auto& s : segX) fix(s);
         for (auto& s : segAX) fix(s);
         for (auto& s : segAY) fix(s);
+        auto flatten = [](const std::vector<Segment<T>>& segs, AnyFold* f) {
+            f->n = 0;
+            int total = 0;
+            for (auto& s : segs) total += s.nin;
+            if (total > kAnyInputs) return;
+            for (auto& s : segs)
+                for (int i = 0; i < s.nin; i++, f->n++) {
+                    f->field[f->n] = (short)s.in[i];
+                    f->out[f->n] = (short)s.out[0];
+                    f->last[f->n] = i + 1 == s.nin;
+                    f->coef[f->n] = s.coef[0][i];
+                }
+        };
+        flatten(segY, &c->anyY);
+        flatten(segX, &c->anyX);
+        flatten(segAX, &c->anyAX);
+        flatten(segAY, &c->anyAY);
         if (!segY.empty()) std::memcpy(host.data() + c->off_segY, segY.data(), sizeof(Segment<T>) * segY.size());
         if (!segAX.empty()) std::memcpy(host.data() + c->off_segAX, segAX.data(), sizeof(Segment<T>) * segAX.size());
         if (!segAY.empty()) std::memcpy(host.data() + c->off_segAY, segAY.data(), sizeof(Segment<T>) * segAY.size());
@@ -725,6 +751,25 @@ template <typename T> struct Impl {
         return tstop(c, kind, st, t0);
     }
 
+    // y or x pass (axis d) on the runtime-length kernels; *done is false when they do not cover it.  They take the
+    // lengths without a compile-time kernel (measured against the general kernels, us: y pass 101 against 715 and x
+    // pass 41 against 252 at 150x135x75; against the compile-time ones they lose, 1940 to 1014 for the y pass at
+    // 512x512x104); what they do not cover, a prime factor above 17 or a tile beyond shared memory, stays on the
+    // general kernels.
+    static int any_axis(qpd_ctx* c, const AxisArgs<T>& a, int d, const AnyFold& f, AnyMode mode, int kind,
+                        cudaStream_t st, bool* done) {
+        *done = false;
+        if (!c->fast || !c->any_ok[d] || f.n == 0 || c->n > 0x7fffffffLL) return QPD_OK;
+        cudaEvent_t t0;
+        QPD_TRY(tstart(c, st, &t0));
+        // pencils of the y pass are (x, z), z contiguous; those of the x pass are the whole (y, z) plane
+        QPD_CU(c, launch_axis_any<T>(a, f, c->any[d], mode, d == 1 ? c->nx : 1, d == 1 ? c->nz : c->ny * c->nz, c->sms,
+                                     c->smem_max, st, done));
+        if (*done) return tstop(c, kind, st, t0);
+        if (t0) c->pool.push_back(t0);
+        return QPD_OK;
+    }
+
     template <int EPI> static int run_axis(qpd_ctx* c, AxisArgs<T>& a, int64_t nouter, int kind, cudaStream_t st) {
         const size_t lim = max_smem(c);
         int best = -1, bestCz = 0;
@@ -779,6 +824,9 @@ template <typename T> struct Impl {
                 if (a.N == 512) return adj_tma_<512, 512, Radix<8, 8, 8>>(c, a, nouter, xp, st, nfields_in);
             }
         }
+        bool done = false;
+        QPD_TRY(any_axis(c, a, xp ? 0 : 1, xp ? c->anyAX : c->anyAY, AnyMode::Pre, QPD_K_ADJAXIS, st, &done));
+        if (done) return QPD_OK;
         const size_t lim = max_smem(c);
         int best = -1, bestCz = 0;
         for (int i = 0; i < 4; i++) {
@@ -1195,6 +1243,7 @@ template <typename T> struct Impl {
                 }
             }
         }
+        if (!seeded) QPD_TRY(any_axis(c, x, 0, c->anyX, AnyMode::Seed, QPD_K_ADJSEED, st, &seeded));
         if (!seeded) QPD_TRY(run_axis<2>(c, x, c->ny, QPD_K_ADJSEED, st));
 
         AxisArgs<T> ax;
@@ -1244,7 +1293,26 @@ template <typename T> struct Impl {
                 if (c->nz == 104) return adj_z_fast_<104, 8, 256, Pfa<8, 13>>(c, az, st);
             }
         }
+        if (c->fast && c->any_ok[2]) {
+            bool done = false;
+            cudaEvent_t t0;
+            QPD_TRY(tstart(c, st, &t0));
+            QPD_CU(c, launch_adjz_any<T>(az, c->any[2], c->sms, c->smem_max, st, &done));
+            if (done) return tstop(c, QPD_K_ADJZ, st, t0);
+            if (t0) c->pool.push_back(t0);
+        }
         return run_adj_z(c, az, st);
+    }
+
+    static int any_z(qpd_ctx* c, const ZArgs<T>& z, cudaStream_t st, bool* done) {
+        *done = false;
+        if (!c->fast || !c->any_ok[2]) return QPD_OK;
+        cudaEvent_t t0;
+        QPD_TRY(tstart(c, st, &t0));
+        QPD_CU(c, launch_z_any<T>(z, c->any[2], c->sms, c->smem_max, st, done));
+        if (*done) return tstop(c, QPD_K_ZSTAGE, st, t0);
+        if (t0) c->pool.push_back(t0);
+        return QPD_OK;
     }
 
     static int forward_zy(qpd_ctx* c, const Inputs<T>& in, cudaStream_t st, bool yfast = false) {
@@ -1262,6 +1330,7 @@ template <typename T> struct Impl {
                 }
             }
             if (!done && c->fast) QPD_TRY(fast_z(c, z, st, &done));
+            if (!done) QPD_TRY(any_z(c, z, st, &done));
             if (!done) QPD_TRY(run_z(c, z, st));
 
             AxisArgs<T> y;
@@ -1293,6 +1362,7 @@ template <typename T> struct Impl {
             }
             done = false;
             if (c->fast) QPD_TRY(fast_axis<false>(c, y, c->nx, QPD_K_YPASS, st, &done));
+            if (!done) QPD_TRY(any_axis(c, y, 1, c->anyY, AnyMode::Store, QPD_K_YPASS, st, &done));
             if (!done) QPD_TRY(run_axis<0>(c, y, c->nx, QPD_K_YPASS, st));
         }
         return QPD_OK;
@@ -1337,6 +1407,7 @@ template <typename T> struct Impl {
             }
             bool done = false;
             if (c->fast) QPD_TRY(fast_axis<true>(c, x, c->ny, QPD_K_XPASS, st, &done));
+            if (!done) QPD_TRY(any_axis(c, x, 0, c->anyX, AnyMode::Intensity, QPD_K_XPASS, st, &done));
             if (done) return QPD_OK;
             return run_axis<1>(c, x, c->ny, QPD_K_XPASS, st);
         }
@@ -1624,6 +1695,27 @@ int upload_twiddles(qpd_ctx* c, int d, int64_t N) {
     return QPD_OK;
 }
 
+// Stages and twiddle rows of an axis for the runtime-length passes.
+int plan_any(qpd_ctx* c, int d, int64_t N) {
+    c->any[d] = AnyStages();
+    c->any_ok[d] = any_stages(N, &c->any[d]);
+    const size_t k = c->any[d].ntw;
+    if (!c->any_ok[d] || k == 0) return QPD_OK;
+    std::vector<double2> w(k);
+    any_twiddles(c->any[d], w.data());
+    if (c->precision == QPD_FP64) {
+        QPD_TRY(dev_reserve(c, c->tw_any[d], sizeof(double2) * k, "twiddle rows"));
+        QPD_CU(c, cudaMemcpy(c->tw_any[d].p, w.data(), sizeof(double2) * k, cudaMemcpyHostToDevice));
+    } else {
+        std::vector<float2> f(k);
+        for (size_t m = 0; m < k; m++) f[m] = make_float2((float)w[m].x, (float)w[m].y);
+        QPD_TRY(dev_reserve(c, c->tw_any[d], sizeof(float2) * k, "twiddle rows"));
+        QPD_CU(c, cudaMemcpy(c->tw_any[d].p, f.data(), sizeof(float2) * k, cudaMemcpyHostToDevice));
+    }
+    c->any[d].tw = c->tw_any[d].p;
+    return QPD_OK;
+}
+
 // The butterflies' unit roots, once per device (constant memory is per device and module).
 int roots_init(qpd_ctx* c) {
     static std::mutex mu;
@@ -1758,6 +1850,8 @@ int qpd_create(int device, uint64_t hbm_budget_bytes, qpd_ctx** out) {
     c->fast = !(gen && gen[0] == '1');
     const char* notma = std::getenv("QPOP_B200_NO_TMA");
     c->tma = !(notma && notma[0] == '1');
+    cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
+    c->smem_max = max_smem(c);
     if (const char* k = std::getenv("QPOP_B200_ZCFG")) c->knob_z = std::atoi(k);
     if (const char* k = std::getenv("QPOP_B200_NBUF")) c->knob_nbuf = std::atoi(k) == 3 ? 3 : 2;
     if (const char* k = std::getenv("QPOP_B200_ZPFA")) c->knob_zpfa = std::atoi(k);
@@ -1790,7 +1884,7 @@ int qpd_destroy(qpd_ctx* c) {
     if (!c) return QPD_OK;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (DevMem* m : {&c->tw[0], &c->tw[1], &c->tw[2], &c->tables, &c->fields, &c->adjw, &c->packed, &c->dense,
+    for (DevMem* m : {&c->tw[0], &c->tw[1], &c->tw[2], &c->tw_any[0], &c->tw_any[1], &c->tw_any[2], &c->tables, &c->fields, &c->adjw, &c->packed, &c->dense,
                       &c->stage, &c->Idev, &c->flags, &c->status})
         dev_free(c, *m);
     c->workers.reset();
@@ -1858,6 +1952,7 @@ int qpd_plan(qpd_ctx* c, const qpd_grid* g, int32_t nPhase, int32_t nStruc, int3
         c->radix[d] = N[d] > 1 ? factorise(N[d]) : std::vector<int>();
         if ((int)c->radix[d].size() > kMaxStages) return fail(c, QPD_ERR_UNSUPPORTED, "axis %d has too many stages", d);
         QPD_TRY(upload_twiddles(c, d, N[d]));
+        QPD_TRY(plan_any(c, d, N[d]));
     }
     c->planned = true;
     return QPD_OK;
