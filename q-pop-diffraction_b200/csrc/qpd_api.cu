@@ -18,6 +18,7 @@
 
 #include "qpopdiff.h"
 #include "qpd_any.h"
+#include "qpd_axisct.h"
 #include "qpd_fast.cuh"
 #include "qpd_fields.cuh"
 #include "qpd_zpfa.cuh"
@@ -58,7 +59,6 @@ struct qpd_ctx {
     int nPhase = 0, nStruc = 0, precision = QPD_FP32, schedule = QPD_SCHED_FUSED;
     std::vector<int> radix[3];
     DevMem tw[3];
-    DevMem tw_any[3];  // the same in the order of the runtime-length passes (AnyStages)
 
     // crystal
     bool have_crystal = false;
@@ -84,6 +84,7 @@ struct qpd_ctx {
     qpd::AnyStages any[3];
     bool any_ok[3] = {false, false, false};
     qpd::AnyFold anyY, anyX, anyAX, anyAY;
+    qpd::AxisCtShape ct[3];  // compile-time y and x passes of the float32 path (cz = 0: none); tw: their twiddle rows
     int sms = 0;
     size_t smem_max = 0;
 
@@ -751,6 +752,31 @@ template <typename T> struct Impl {
         return tstop(c, kind, st, t0);
     }
 
+    // y or x pass (axis d) on the compile-time register-folding kernels; nfields: fields of the buffer at a.in.
+    // They take every power-of-two length that they have (us, axis_tma -> axis_ct): y pass 1015 -> 745 and x pass
+    // 397 -> 306 at 512x512x104, 3870 -> 2867 and 1577 -> 996 at 1024x1024x68, 167 -> 110 and 74 -> 58 at 256x256x64,
+    // 86 -> 67 and 39 -> 35 at 128^3; the adjoint's x and y passes 395 -> 164 at 256x256x64.
+    static int ct_axis(qpd_ctx* c, const AxisArgs<T>& a, int d, const AnyFold& f, AnyMode mode, int64_t nfields, int kind,
+                       cudaStream_t st, bool* done) {
+        *done = false;
+        if constexpr (sizeof(T) == 4) {
+            const AxisCtShape& s = c->ct[d];
+            // the map's row strides are multiples of 16 bytes for even nz; a launch shape chosen for axis_tma keeps it
+            if (!c->fast || !c->tma || c->knob_oop != 1 || c->knob_nbuf != 2 || (kind >= QPD_K_ADJSEED && !c->knob_adj_tma) ||
+                s.cz == 0 || f.n == 0 || a.nz % 2 != 0 || a.accumulate)
+                return QPD_OK;
+            CUtensorMap map;
+            QPD_TRY(field_map(c, &map, const_cast<C*>(a.in), false, a.nz, c->ny, nfields * c->nx, 2 * s.cz,
+                              d == 0 ? 1 : s.box, d == 0 ? s.box : 1));
+            cudaEvent_t t0;
+            QPD_TRY(tstart(c, st, &t0));
+            QPD_CU(c, launch_axis_ct(map, a, f, static_cast<const C*>(s.stages.tw), mode, d == 0, d == 0 ? c->ny : c->nx, st));
+            *done = true;
+            return tstop(c, kind, st, t0);
+        }
+        return QPD_OK;
+    }
+
     // y or x pass (axis d) on the runtime-length kernels; *done is false when they do not cover it.  They take the
     // lengths without a compile-time kernel (measured against the general kernels, us: y pass 101 against 715 and x
     // pass 41 against 252 at 150x135x75; against the compile-time ones they lose, 1940 to 1014 for the y pass at
@@ -818,13 +844,16 @@ template <typename T> struct Impl {
 
     static int run_adj_axis(qpd_ctx* c, AxisArgs<T>& a, int64_t nouter, cudaStream_t st, bool xp = false,
                             int64_t nfields_in = 0) {
+        bool done = false;
+        if (nfields_in > 0)
+            QPD_TRY(ct_axis(c, a, xp ? 0 : 1, xp ? c->anyAX : c->anyAY, AnyMode::Pre, nfields_in, QPD_K_ADJAXIS, st, &done));
+        if (done) return QPD_OK;
         if constexpr (sizeof(T) == 4) {
             if (c->fast && c->tma && c->knob_adj_tma && nfields_in > 0 && a.nz % 2 == 0) {
                 if (a.N == 256) return adj_tma_<256, 256, Radix<8, 8, 4>>(c, a, nouter, xp, st, nfields_in);
                 if (a.N == 512) return adj_tma_<512, 512, Radix<8, 8, 8>>(c, a, nouter, xp, st, nfields_in);
             }
         }
-        bool done = false;
         QPD_TRY(any_axis(c, a, xp ? 0 : 1, xp ? c->anyAX : c->anyAY, AnyMode::Pre, QPD_K_ADJAXIS, st, &done));
         if (done) return QPD_OK;
         const size_t lim = max_smem(c);
@@ -1229,8 +1258,9 @@ template <typename T> struct Impl {
         x.out = W;
         x.gI = dI;
         bool seeded = false;
+        QPD_TRY(ct_axis(c, x, 0, c->anyX, AnyMode::Seed, 3 * c->ng1, QPD_K_ADJSEED, st, &seeded));
         if constexpr (sizeof(T) == 4) {
-            if (c->fast && c->tma && c->knob_adj_tma && c->nz % 2 == 0) {
+            if (!seeded && c->fast && c->tma && c->knob_adj_tma && c->nz % 2 == 0) {
                 using namespace qpd;
                 if (c->nx == 256) {
                     QPD_TRY((tma_axis_b<256, 8, 256, 2, true, true, Radix<8, 8, 4>, 2, true, false, false, true>(
@@ -1360,8 +1390,8 @@ template <typename T> struct Impl {
                     return bulk_axis_<4000, 256, Radix<8, 4, 5, 5, 5>>(c, y, st);
                 }
             }
-            done = false;
-            if (c->fast) QPD_TRY(fast_axis<false>(c, y, c->nx, QPD_K_YPASS, st, &done));
+            QPD_TRY(ct_axis(c, y, 1, c->anyY, AnyMode::Store, 3 * c->ng1, QPD_K_YPASS, st, &done));
+            if (c->fast && !done) QPD_TRY(fast_axis<false>(c, y, c->nx, QPD_K_YPASS, st, &done));
             if (!done) QPD_TRY(any_axis(c, y, 1, c->anyY, AnyMode::Store, QPD_K_YPASS, st, &done));
             if (!done) QPD_TRY(run_axis<0>(c, y, c->nx, QPD_K_YPASS, st));
         }
@@ -1406,7 +1436,8 @@ template <typename T> struct Impl {
                 }
             }
             bool done = false;
-            if (c->fast) QPD_TRY(fast_axis<true>(c, x, c->ny, QPD_K_XPASS, st, &done));
+            QPD_TRY(ct_axis(c, x, 0, c->anyX, AnyMode::Intensity, 3 * c->ng1, QPD_K_XPASS, st, &done));
+            if (c->fast && !done) QPD_TRY(fast_axis<true>(c, x, c->ny, QPD_K_XPASS, st, &done));
             if (!done) QPD_TRY(any_axis(c, x, 0, c->anyX, AnyMode::Intensity, QPD_K_XPASS, st, &done));
             if (done) return QPD_OK;
             return run_axis<1>(c, x, c->ny, QPD_K_XPASS, st);
@@ -1677,42 +1708,32 @@ template <typename T> struct Impl {
     }
 };
 
+// The tables of an axis in one buffer: exp(-2 pi i m / N) for m < N, then the twiddle rows of the runtime-length
+// passes and of the compile-time ones, each where a 16-byte load can start.
 int upload_twiddles(qpd_ctx* c, int d, int64_t N) {
-    std::vector<double2> w(N);
+    c->any[d] = AnyStages();
+    c->any_ok[d] = any_stages(N, &c->any[d]);
+    c->ct[d] = AxisCtShape();
+    if (c->precision == QPD_FP32 && d < 2) c->ct[d] = axis_ct_shape(N);
+    const size_t at_any = (N + 1) / 2 * 2, at_ct = at_any + (c->any_ok[d] ? c->any[d].ntw : 0);
+    std::vector<double2> w(at_ct + c->ct[d].stages.ntw, make_double2(0.0, 0.0));
     for (int64_t m = 0; m < N; m++) {
         const double a = 2.0 * M_PI * (double)m / (double)N;
         w[m] = make_double2(std::cos(a), -std::sin(a));
     }
+    if (c->any_ok[d]) any_twiddles(c->any[d], w.data() + at_any);
+    if (c->ct[d].cz) any_twiddles(c->ct[d].stages, w.data() + at_ct);
+    const size_t el = c->precision == QPD_FP64 ? sizeof(double2) : sizeof(float2);
+    QPD_TRY(dev_reserve(c, c->tw[d], el * w.size(), "twiddles"));
     if (c->precision == QPD_FP64) {
-        QPD_TRY(dev_reserve(c, c->tw[d], sizeof(double2) * N, "twiddles"));
-        QPD_CU(c, cudaMemcpy(c->tw[d].p, w.data(), sizeof(double2) * N, cudaMemcpyHostToDevice));
+        QPD_CU(c, cudaMemcpy(c->tw[d].p, w.data(), el * w.size(), cudaMemcpyHostToDevice));
     } else {
-        std::vector<float2> f(N);
-        for (int64_t m = 0; m < N; m++) f[m] = make_float2((float)w[m].x, (float)w[m].y);
-        QPD_TRY(dev_reserve(c, c->tw[d], sizeof(float2) * N, "twiddles"));
-        QPD_CU(c, cudaMemcpy(c->tw[d].p, f.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
+        std::vector<float2> f(w.size());
+        for (size_t m = 0; m < w.size(); m++) f[m] = make_float2((float)w[m].x, (float)w[m].y);
+        QPD_CU(c, cudaMemcpy(c->tw[d].p, f.data(), el * w.size(), cudaMemcpyHostToDevice));
     }
-    return QPD_OK;
-}
-
-// Stages and twiddle rows of an axis for the runtime-length passes.
-int plan_any(qpd_ctx* c, int d, int64_t N) {
-    c->any[d] = AnyStages();
-    c->any_ok[d] = any_stages(N, &c->any[d]);
-    const size_t k = c->any[d].ntw;
-    if (!c->any_ok[d] || k == 0) return QPD_OK;
-    std::vector<double2> w(k);
-    any_twiddles(c->any[d], w.data());
-    if (c->precision == QPD_FP64) {
-        QPD_TRY(dev_reserve(c, c->tw_any[d], sizeof(double2) * k, "twiddle rows"));
-        QPD_CU(c, cudaMemcpy(c->tw_any[d].p, w.data(), sizeof(double2) * k, cudaMemcpyHostToDevice));
-    } else {
-        std::vector<float2> f(k);
-        for (size_t m = 0; m < k; m++) f[m] = make_float2((float)w[m].x, (float)w[m].y);
-        QPD_TRY(dev_reserve(c, c->tw_any[d], sizeof(float2) * k, "twiddle rows"));
-        QPD_CU(c, cudaMemcpy(c->tw_any[d].p, f.data(), sizeof(float2) * k, cudaMemcpyHostToDevice));
-    }
-    c->any[d].tw = c->tw_any[d].p;
+    c->any[d].tw = static_cast<unsigned char*>(c->tw[d].p) + el * at_any;
+    c->ct[d].stages.tw = static_cast<unsigned char*>(c->tw[d].p) + el * at_ct;
     return QPD_OK;
 }
 
@@ -1884,7 +1905,7 @@ int qpd_destroy(qpd_ctx* c) {
     if (!c) return QPD_OK;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (DevMem* m : {&c->tw[0], &c->tw[1], &c->tw[2], &c->tw_any[0], &c->tw_any[1], &c->tw_any[2], &c->tables, &c->fields, &c->adjw, &c->packed, &c->dense,
+    for (DevMem* m : {&c->tw[0], &c->tw[1], &c->tw[2], &c->tables, &c->fields, &c->adjw, &c->packed, &c->dense,
                       &c->stage, &c->Idev, &c->flags, &c->status})
         dev_free(c, *m);
     c->workers.reset();
@@ -1952,7 +1973,6 @@ int qpd_plan(qpd_ctx* c, const qpd_grid* g, int32_t nPhase, int32_t nStruc, int3
         c->radix[d] = N[d] > 1 ? factorise(N[d]) : std::vector<int>();
         if ((int)c->radix[d].size() > kMaxStages) return fail(c, QPD_ERR_UNSUPPORTED, "axis %d has too many stages", d);
         QPD_TRY(upload_twiddles(c, d, N[d]));
-        QPD_TRY(plan_any(c, d, N[d]));
     }
     c->planned = true;
     return QPD_OK;
