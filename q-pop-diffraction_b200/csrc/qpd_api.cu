@@ -21,6 +21,7 @@
 #include "qpd_axisct.h"
 #include "qpd_fast.cuh"
 #include "qpd_fields.cuh"
+#include "qpd_zcol.h"
 #include "qpd_zpfa.cuh"
 #include "qpd_host.h"
 #include "qpd_kernels.cuh"
@@ -70,6 +71,8 @@ struct qpd_ctx {
     double scale2 = 0;
     DevMem tables;                     // complex coefficient tables, shape factors, constants, segments
     // offsets into `tables`
+    size_t off_iso = 0;
+    bool iso = false;                  // every ionic shift is a multiple of P: su[d][s] = k delta_ds
     size_t off_apc = 0, off_coefE = 0, off_coefUz = 0, off_S[3] = {0, 0, 0}, off_segY = 0, off_segX = 0;
     size_t off_pex = 0, off_pey = 0, off_pez = 0, off_k[3] = {0, 0, 0};
     int nsegY = 0;
@@ -440,6 +443,16 @@ template <typename T> struct Impl {
                     e.fi = (T)k->f_im[p * A + a];
                 }
         }
+        // su[d][s] = k delta_ds for every phase and atom: the phase argument needs k alone
+        c->iso = NS == 3;
+        c->off_iso = place(sizeof(double) * NP * A);
+        for (int p = 0; p < NP; p++)
+            for (int i = 0; i < A; i++) {
+                auto su = [&](int d, int s) { return k->su[((d * NS + s) * NP + p) * A + order[i]]; };
+                for (int d = 0; d < 3 && c->iso; d++)
+                    for (int s = 0; s < 3; s++) c->iso = c->iso && su(d, s) == (d == s ? su(0, 0) : 0.0);
+                if (c->iso) reinterpret_cast<double*>(host.data() + c->off_iso)[p * A + i] = su(0, 0);
+            }
         for (int d = 0; d < 3; d++) {
             c->off_S[d] = place(sizeof(double) * N[d]);
             std::memcpy(host.data() + c->off_S[d], S[d].data(), sizeof(double) * N[d]);
@@ -989,6 +1002,17 @@ template <typename T> struct Impl {
         *done = true;
         constexpr bool F = sizeof(T) == 4;
         if constexpr (F) {
+            // single-phase inputs of a covered nz (us, before -> after): 1826 -> 1530 at 512x512x104, 4457 -> 3980 at
+            // 1024x1024x68, 238 -> 187 at 256x256x64, 144 -> 116 at 128^3.  A z stage chosen by a switch keeps it, and
+            // both routes of the y-fastest grid keep the arithmetic of that route's z stage (zstage_pfa).
+            if (c->knob_zpfa < 0 && c->knob_z == 0 && c->knob_zregin == 1 && !yfast_grid(c)) {
+                cudaEvent_t t0;
+                QPD_TRY(tstart(c, st, &t0));
+                QPD_CU(c, launch_zcol(a, c->cta_tiles, c->sms, c->smem_max, st, done));
+                if (*done) return tstop(c, QPD_K_ZSTAGE, st, t0);
+                if (t0) c->pool.push_back(t0);
+                *done = true;
+            }
             // single-phase inputs: the register-fused prime-factor z stage
             if (c->tma && !a.in.wdense && a.nAtom <= 16) {
                 if (a.nz == 104 && c->knob_zpfa == 1 &&
@@ -1086,11 +1110,12 @@ template <typename T> struct Impl {
         return tstop(c, QPD_K_YPASS, st, t0);
     }
 
+    static bool yfast_grid(const qpd_ctx* c) { return c->nx == 4000 && c->ny == 4000 && c->nz == 68; }
+
     // The 4000 x 4000 x 68 route: fused z stage writing y-fastest fields, bulk y pass, swapped x pass.
     static bool yfast_ok(qpd_ctx* c, const Inputs<T>& in) {
         if constexpr (sizeof(T) != 4) return false;
-        return c->knob_yfast && c->fast && c->tma && c->knob_zpfa != 0 && !in.wdense && c->nAtom <= 16 &&
-               c->nx == 4000 && c->ny == 4000 && c->nz == 68 &&
+        return c->knob_yfast && c->fast && c->tma && c->knob_zpfa != 0 && !in.wdense && c->nAtom <= 16 && yfast_grid(c) &&
                ZPfaLayout<T, 4, 17>::bytes(in.nPhase * c->nAtom, c->nAtom) <= max_smem(c);
     }
 
@@ -1214,6 +1239,7 @@ template <typename T> struct Impl {
         z.nz = (int)c->nz;
         z.nAtom = c->nAtom;
         z.apc = tab<AtomPhase<T>>(c, c->off_apc);
+        z.isok = c->iso ? tab<double>(c, c->off_iso) : nullptr;
         z.coefE = tab<C>(c, c->off_coefE);
         z.coefUz = tab<C>(c, c->off_coefUz);
         for (int i = 0; i < c->nAtom; i++) z.grp[i] = c->grp[i];

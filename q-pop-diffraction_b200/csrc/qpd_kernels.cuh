@@ -181,6 +181,7 @@ template <typename T> struct ZArgs {
     AxisPlan zp;
     int* status;                  // device status word: bounded waits record timeouts here
     long long ny;                 // yfast: the y extent
+    const double* isok;           // k of every (phase, atom) when all ionic shifts are k times P, else null
     int yfast;                    // fields y fastest (zstage_pfa only): 1 (x, k_z, y), 2 (k_z, x, y)
 };
 

@@ -1,6 +1,7 @@
 """
-The compile-time y and x passes (csrc/qpd_axisct.cuh) of the float32 path, at the edges of their tiles: whole and
-partial z chunks, one to three outer indices.
+The compile-time z stage (csrc/qpd_zcol.cuh) and y and x passes (csrc/qpd_axisct.cuh) of the float32 path, at the
+edges of their tiles: column counts that a tile does not divide, z extents that leave a partial chunk, isotropic and
+general ionic shifts, one to three phases, cells that do not scatter, fractional weights.
 
 Tolerances: the float32 contract against the oracle (max |dI| / I_max <= 1e-5, relative error <= 1e-3 above
 1e-6 I_max); between these kernels and the general ones both errors add: 2e-5 of the largest value.
@@ -29,6 +30,21 @@ def plan_of(case):
     plan = Plan(case.shape, (p.dx, p.dy, p.dz), p.nPhase, p.nStruc)
     plan.set_crystal(crystal_from(p, case.atoms))
     return plan
+
+
+@pytest.mark.parametrize("iso", [True, False])
+@pytest.mark.parametrize("nz", [32, 64, 68, 104, 128])
+def test_z_stage(gpu, nz, iso):
+    from oracle import diffraction_oracle as oracle
+    for shape, phases, weights in (((1, 1, nz), 1, "onehot"), ((3, 5, nz), 2, "region"), ((7, 9, nz), 3, "onehot")):
+        case = make_case(shape, phases, weights, iso, seed=sum(shape))
+        ref = oracle.diffraction(*case.args())[0]
+        with plan_of(case) as plan:
+            plan.set_cta_tiles(2 if phases == 3 else 0)
+            I = plan.run_host(case.oPhase, case.oStruc, case.u, case.region)
+            plan.device_status()
+        dmax, rel = fp32_errors(I, ref)
+        assert dmax <= 1e-5 and rel <= 1e-3, (shape, dmax, rel)
 
 
 @pytest.mark.parametrize("N", [64, 128, 256, 512, 1024])
