@@ -95,10 +95,21 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
     C acc[EPT];
 #pragma unroll
     for (int e = 0; e < EPT; e++) acc[e] = make_float2(0.f, 0.f);
+#pragma unroll 1
     for (int i = 0; i < f.n; i++) {
         C* const cur = tiles + (i % RING) * TILE;
         C* const W = tiles + (R3 > 1 ? 2 : (i + 2) % 3) * TILE;
         const C* const cf = static_cast<const C*>(f.coef[i]);
+        // with 16 values per thread the fold's coefficients are requested before the input's tile is awaited (1024
+        // points: y pass 2850 -> 2290 us at 1024x1024x68); with 8, at 64 registers, they would spill
+        constexpr bool EARLY = EPT > 8 && MODE != AnyMode::Pre;
+        C cfr[EARLY ? EPT : 1];
+        if constexpr (EARLY) {
+#pragma unroll
+            for (int q = 0; q < EPT / RL; q++)
+#pragma unroll
+                for (int s = 0; s < RL; s++) cfr[q * RL + s] = __ldg(cf + j0 + q * JT + s * (N / RL));
+        }
         const bool ok = mbar_wait(&bar[i & 1], (i >> 1) & 1, a.status);
         // ---- stage 1
         {
@@ -177,7 +188,7 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
             for (int s = 0; s < RL; s++) {
                 const int e = q * RL + s;
                 if constexpr (MODE == AnyMode::Pre) acc[e] = x[e];
-                else fold_fma(acc[e], __ldg(cf + j0 + q * JT + s * (N / RL)), x[e]);
+                else fold_fma(acc[e], EARLY ? cfr[EARLY ? e : 0] : __ldg(cf + j0 + q * JT + s * (N / RL)), x[e]);
             }
         if (!f.last[i]) continue;
         if (live) {
@@ -193,6 +204,16 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
                 const int sy = fftshift_at(ky, ny), sz = fftshift_at(kz, a.nz);
                 const double syz = a.S[1][ky] * a.S[2][kz];
                 C* const dst = a.out + (long long)f.out[i] * a.fstride + base;
+                double gi[MODE == AnyMode::Seed ? EPT : 1];
+                if constexpr (MODE == AnyMode::Seed) {  // all in flight before the first is needed
+#pragma unroll
+                    for (int q = 0; q < EPT / RL; q++)
+#pragma unroll
+                        for (int s = 0; s < RL; s++) {
+                            const int k = j0 + q * JT + s * (N / RL);
+                            gi[q * RL + s] = __ldg(a.gI + ((long long)(k < N / 2 ? k + N / 2 : k - N / 2) * ny + sy) * a.nz + sz);
+                        }
+                }
 #pragma unroll
                 for (int q = 0; q < EPT / RL; q++)
 #pragma unroll
@@ -205,7 +226,7 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
                             a.I[at] = floor_1e50(S * S * (re * re + im * im) * a.scale2);
                         } else {
                             const double S2 = S * S * a.scale2;
-                            const double g = S2 * (re * re + im * im) > 1e-50 ? a.gI[at] * S2 : 0.0;
+                            const double g = S2 * (re * re + im * im) > 1e-50 ? gi[MODE == AnyMode::Seed ? e : 0] * S2 : 0.0;
                             dst[k * a.stride] = make_float2((float)(g * re), (float)(-g * im));
                         }
                     }
