@@ -20,7 +20,7 @@
 #include "qpd_any.h"
 #include "qpd_axisct.h"
 #include "qpd_fast.cuh"
-#include "qpd_fields.cuh"
+#include "qpd_fields.h"
 #include "qpd_zcol.h"
 #include "qpd_zpfa.cuh"
 #include "qpd_host.h"
@@ -1867,13 +1867,9 @@ int pack_fields_t(qpd_ctx* c, const qpd_fields* in, void* P, void* U, int8_t* ph
     a.weight = static_cast<T*>(weight);
     a.wdense = static_cast<T*>(wdense);
     a.flags = fd;
-    const int planes = c->nStruc + (in->u[0] ? 3 : 0) + (in->phase ? c->nPhase : 0) + (in->region ? 1 : 0);
-    const size_t smem = fields_smem_bytes(planes);
-    QPD_CU(c, cudaFuncSetAttribute(fields_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaEvent_t t0;
     QPD_TRY(tstart(c, st, &t0));
-    dim3 grid((unsigned)((c->nx + kFT - 1) / kFT), (unsigned)c->ny);
-    fields_kernel<T><<<grid, dim3(kFT, kFRows), smem, st>>>(a);
+    QPD_CU(c, launch_fields<T>(a, st));
     return tstop(c, QPD_K_PACK, st, t0);
 }
 
