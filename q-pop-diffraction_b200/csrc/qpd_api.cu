@@ -1003,7 +1003,8 @@ template <typename T> struct Impl {
         constexpr bool F = sizeof(T) == 4;
         if constexpr (F) {
             // single-phase inputs of a covered nz (us, before -> after): 1826 -> 1530 at 512x512x104, 4457 -> 3980 at
-            // 1024x1024x68, 238 -> 187 at 256x256x64, 144 -> 116 at 128^3.  A z stage chosen by a switch keeps it, and
+            // 1024x1024x68, 238 -> 187 at 256x256x64, 144 -> 116 at 128^3, and against the runtime-length z stage 159 -> 98
+            // at 150x135x75, 74 -> 48 at 120x100x50.  A z stage chosen by a switch keeps it, and
             // both routes of the y-fastest grid keep the arithmetic of that route's z stage (zstage_pfa).
             if (c->knob_zpfa < 0 && c->knob_z == 0 && c->knob_zregin == 1 && !yfast_grid(c)) {
                 cudaEvent_t t0;
@@ -1597,7 +1598,21 @@ template <typename T> struct Impl {
         }
         for (auto& e : c->ring_ev)
             if (!e) QPD_CU(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        const int64_t C = std::min<int64_t>(n, (int64_t)1 << 21);  // cells per chunk
+        // Pageable arrays (NumPy's) cross a device copy through the driver's own staging, one thread at about
+        // 10 GB/s, where the workers read them at several times that and the packed chunk is pinned: every chunk is
+        // packed on the host then, in at least 4 chunks so that the copies overlap the packing (a 96x96x64 call took 4.7 ms the driver's way and
+        // takes 1.1 ms, with the result coming back through the ring below).
+        auto pageable = [](const void* p) {
+            cudaPointerAttributes at;
+            if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+                cudaGetLastError();
+                return true;
+            }
+            return at.type == cudaMemoryTypeUnregistered;
+        };
+        const bool paged = pageable(oPhase) || pageable(u) || (NS > 0 && pageable(oStruc)) || (region && pageable(region));
+        int64_t C = std::min<int64_t>(n, (int64_t)1 << 21);  // cells per chunk
+        if (paged) C = std::min<int64_t>(C, std::max<int64_t>((int64_t)1 << 16, ((n + 3) / 4 + 63) / 64 * 64));
         constexpr int NSLOT = 3;
         // Chunks take one of two routes that run at the same time: the host workers pack a chunk
         // (fewer bytes on the link, host memory bandwidth spent) or it crosses the link as float64
@@ -1606,7 +1621,7 @@ template <typename T> struct Impl {
         // the host packs, and a slow host packs fewer chunks (QPOP_B200_ROUTE_DEPTH sets that queue
         // depth, default 1).  QPOP_B200_HOST_SHARE fixes the share
         // of host-packed chunks instead (0: all device, 1: all host).
-        double share = -1.0;
+        double share = paged ? 1.0 : -1.0;
         if (const char* e = std::getenv("QPOP_B200_HOST_SHARE")) share = std::min(1.0, std::max(0.0, std::atof(e)));
         int depth = 1;  // device route while fewer than `depth` chunks wait on the copy engine
         if (const char* e = std::getenv("QPOP_B200_ROUTE_DEPTH")) depth = std::max(1, std::atoi(e));
@@ -1679,7 +1694,7 @@ template <typename T> struct Impl {
                 const int s = (int)(hosted++ % NSLOT);
                 if (c->ring_busy[s]) QPD_CU(c, cudaEventSynchronize(c->ring_ev[s]));
                 const qpd::HostChunk<T> h = qpd::HostChunk<T>::at(static_cast<unsigned char*>(c->hring) + s * slot, C);
-                const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(c->workers->size() + 1, cnt >> 16));
+                const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(c->workers->size() + 1, cnt >> 13));
                 std::atomic<uint32_t> fl{0};
                 c->workers->parallel(parts, [&](int t) {
                     const int64_t i0 = cnt * t / parts, i1 = cnt * (t + 1) / parts;
@@ -1687,9 +1702,12 @@ template <typename T> struct Impl {
                 });
                 const uint32_t f = fl.load();
                 flags |= f;
-                for (int k = 0; k < 3; k++) {
-                    QPD_CU(c, cudaMemcpyAsync(P + k * n + g0, h.P + k * C, sizeof(T) * cnt, cudaMemcpyHostToDevice, st));
-                    QPD_CU(c, cudaMemcpyAsync(U + k * n + g0, h.U + k * C, sizeof(T) * cnt, cudaMemcpyHostToDevice, st));
+                // the 3 planes of P and the 3 of U follow one another on both sides
+                if (sizeof(T) * (size_t)n <= (size_t)0x7fffffff) {  // a 2-D copy's pitch is at most 2^31 - 1 bytes
+                    QPD_CU(c, cudaMemcpy2DAsync(P + g0, sizeof(T) * n, h.P, sizeof(T) * C, sizeof(T) * cnt, 6, cudaMemcpyHostToDevice, st));
+                } else {
+                    for (int k = 0; k < 6; k++)
+                        QPD_CU(c, cudaMemcpyAsync(P + k * n + g0, h.P + k * C, sizeof(T) * cnt, cudaMemcpyHostToDevice, st));
                 }
                 if (dense) {
                     for (int p = 0; p < NP; p++)
@@ -1727,8 +1745,35 @@ template <typename T> struct Impl {
         }
         double* Id = static_cast<double*>(c->Idev.p);
         QPD_TRY(run_device(c, in, Id, st));
-        QPD_CU(c, cudaMemcpyAsync(I, Id, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-        QPD_CU(c, cudaStreamSynchronize(st));
+        const size_t total = sizeof(double) * n;
+        if (!pageable(I) || c->hring_bytes < NSLOT * (size_t)4096) {
+            QPD_CU(c, cudaMemcpyAsync(I, Id, total, cudaMemcpyDeviceToHost, st));
+            QPD_CU(c, cudaStreamSynchronize(st));
+        } else {
+            // a pageable result comes through the pinned ring, piece by piece, the workers copying (and touching the
+            // pages of) the pieces that have landed
+            const size_t piece = std::min((c->hring_bytes / NSLOT) & ~size_t(4095), std::max<size_t>(((total / 8) & ~size_t(4095)) + 4096, (size_t)1 << 18));
+            const int64_t np = (int64_t)((total + piece - 1) / piece);
+            auto fetch = [&](int64_t i) -> int {
+                const size_t at = i * piece, len = std::min(piece, total - at);
+                QPD_CU(c, cudaMemcpyAsync(static_cast<char*>(c->hring) + (i % NSLOT) * piece, reinterpret_cast<char*>(Id) + at, len, cudaMemcpyDeviceToHost, st));
+                QPD_CU(c, cudaEventRecord(c->ring_ev[i % NSLOT], st));
+                return QPD_OK;
+            };
+            for (int64_t i = 0; i < std::min<int64_t>(np, NSLOT); i++) QPD_TRY(fetch(i));
+            for (int64_t i = 0; i < np; i++) {
+                QPD_CU(c, cudaEventSynchronize(c->ring_ev[i % NSLOT]));
+                const size_t at = i * piece, len = std::min(piece, total - at);
+                const char* src = static_cast<char*>(c->hring) + (i % NSLOT) * piece;
+                const int parts = (int)std::max<size_t>(1, std::min<size_t>(c->workers->size() + 1, len >> 16));
+                c->workers->parallel(parts, [&](int t) {
+                    const size_t a0 = len * t / parts, a1 = len * (t + 1) / parts;
+                    std::memcpy(reinterpret_cast<char*>(I) + at + a0, src + a0, a1 - a0);
+                });
+                if (i + NSLOT < np) QPD_TRY(fetch(i + NSLOT));
+            }
+            QPD_CU(c, cudaStreamSynchronize(st));
+        }
         for (bool& b : c->ring_busy) b = false;
         return check_status(c);
     }
