@@ -35,15 +35,31 @@ cudaError_t pick(const ZArgs<float>& a, int cta_tiles, int sms, size_t smem_max,
 
 }  // namespace
 
+// The lengths from 16 to 136 that are N1 N2 with N1 = 4 .. 8 and N2 = 4 .. 17, each with its cheapest factors (butterflies,
+// a twiddle unless they are coprime).
+#define QPD_ZCOL_LENGTHS(X) \
+    X(4, 4) X(4, 5) X(4, 6) X(4, 7) X(4, 8) X(4, 9) X(4, 11) X(4, 12) X(4, 13) X(4, 15) X(4, 16) X(4, 17) \
+    X(5, 5) X(5, 6) X(5, 7) X(5, 8) X(5, 9) X(5, 10) X(5, 11) X(5, 13) X(5, 14) X(5, 15) X(5, 16) X(5, 17) \
+    X(6, 7) X(6, 9) X(6, 11) X(6, 13) X(6, 15) X(6, 17) \
+    X(7, 7) X(7, 8) X(7, 9) X(7, 11) X(7, 12) X(7, 13) X(7, 14) X(7, 15) X(7, 16) X(7, 17) \
+    X(8, 9) X(8, 11) X(8, 12) X(8, 13) X(8, 15) X(8, 16) X(8, 17)
+
+// Columns per tile: about 128 rows of phase B (four CTAs of four warps per SM), an even number of cells.
+constexpr int zcol_columns(int N1, int N2) {
+    const int a = N1 == 8 ? 2 * N2 : N2, b = 4 * N1;
+    int m = 128 / (a > b ? a : b);
+    if (m < 1) m = 1;
+    return N1 * N2 * m % 2 ? (m > 1 ? m - 1 : 2) : m;
+}
+
 cudaError_t launch_zcol(const ZArgs<float>& a, int cta_tiles, int sms, size_t smem_max, cudaStream_t st, bool* done) {
     *done = false;
     if (a.in.wdense || a.yfast) return cudaSuccess;
     switch (a.nz) {
-        case 32: return pick<4, 8, 16, 3>(a, cta_tiles, sms, smem_max, st, done);
-        case 64: return pick<4, 16, 4, 9>(a, cta_tiles, sms, smem_max, st, done);
-        case 68: return pick<4, 17, 7, 4>(a, cta_tiles, sms, smem_max, st, done);
-        case 104: return pick<8, 13, 4, 4>(a, cta_tiles, sms, smem_max, st, done);
-        case 128: return pick<8, 16, 4, 4>(a, cta_tiles, sms, smem_max, st, done);
+#define QPD_ZCOL_CASE(A, B) \
+    case A * B: return pick<A, B, zcol_columns(A, B), ZCol<A, B, zcol_columns(A, B)>::NT <= 128 ? 4 : 3>(a, cta_tiles, sms, smem_max, st, done);
+        QPD_ZCOL_LENGTHS(QPD_ZCOL_CASE)
+#undef QPD_ZCOL_CASE
     }
     return cudaSuccess;
 }

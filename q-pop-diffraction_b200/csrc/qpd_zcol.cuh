@@ -1,4 +1,4 @@
-// Fused z stage of the float32 schedule for nz = N1 N2 (N1 = 4, or 8 on lane pairs; N2 up to 17) and single-phase
+// Fused z stage of the float32 schedule for nz = N1 N2 (N1 = 4 .. 7, or 8 on lane pairs; N2 up to 17) and single-phase
 // inputs: source, z transform and fold.
 //
 // A column is an N1 x N2 array of cells.  Phase A transforms over the N1 cells of one b in registers, straight
@@ -16,11 +16,11 @@
 //     cell instead of four components) and each lane transforms two of the four components whole;
 //   - cells that do not scatter have a record of zeros, so the sources have no branches;
 //   - with isotropic ionic shifts (su = k delta, ISO) the phase is one fma on qC.P and the shifts are three.
-// Four CTAs of four warps at up to 128 registers beat three of eight at 80, which spill (1.53 against 1.92 ms at
+// Without pairs (N1 = 4 .. 7) a thread holds the N1 cells of its b alone.  Four CTAs of four warps at up to 128 registers beat three of eight at 80, which spill (1.53 against 1.92 ms at
 // 512x512x104, 3.98 against 4.97 at 1024x1024x68).  Folding in phase B's registers and storing from there halves
 // the exchanges but not the wavefronts (1.59 and 4.67 ms).  One B200, us per z stage, before (qpd_fast.cuh, for nz = 68
 // qpd_zpfa.cuh) -> now: 512x512x104 1826 -> 1528, 1024x1024x68 4457 -> 3977, 256x256x64 238 -> 187, 128^3 144 -> 117,
-// 64x64x32 18 -> 15.
+// 64x64x32 18 -> 15; against the runtime-length stage (qpd_any.cuh) 150x135x75 159 -> 98, 120x100x50 74 -> 48.
 #pragma once
 
 #include "qpd_kernels.cuh"
@@ -39,6 +39,7 @@ struct alignas(16) IsoAtom {
 
 template <int N1, int N2, int M> struct ZCol {
     static constexpr int N = N1 * N2, CELLS = M * N;
+    static_assert(CELLS % 2 == 0, "16-byte tables behind the inputs");
     static constexpr int SPLIT = N1 == 8 ? 2 : 1;
     static constexpr bool PFA = zcol_gcd(N1, N2) == 1;
     static constexpr int H = (N2 + 1) / 2;                     // 16-byte units of a row
@@ -74,7 +75,8 @@ __global__ void __launch_bounds__(ZCol<N1, N2, M>::NT, MINB) zcol(const __grid_c
     using L = ZCol<N1, N2, M>;
     using C = float2;
     constexpr int N = L::N, NT = L::NT, RP = L::RP, CP = L::CP, CELLS = L::CELLS, SPLIT = L::SPLIT;
-    static_assert(N1 == 4 || N1 == 8, "phase A holds 4 cells per thread");
+    static_assert(N1 >= 4 && N1 <= 8, "phase A holds 4 to 7 cells per thread");
+    constexpr int CA = SPLIT == 2 ? 4 : N1;  // cells of a phase-A item
     extern __shared__ __align__(16) unsigned char zsm[];
     float4* const inA = reinterpret_cast<float4*>(zsm);          // P, u_x
     float4* const inB = inA + CELLS;                             // u_y, u_z, qC.u / 2 pi (double)
@@ -129,10 +131,10 @@ __global__ void __launch_bounds__(ZCol<N1, N2, M>::NT, MINB) zcol(const __grid_c
     const bool actA = tid < L::IA;
     const int cell0 = actA ? am * N + 4 * ah * N2 + ab : 0;
     C* const st0 = xb + (actA ? (am * 4 + (SPLIT == 2 ? 2 * ah : 0)) * CP + ab : 0);
-    C tw4[3] = {};  // N1 = 4: exp(-2 pi i b k / N), k = 1..3
+    C twa[N1 - 1] = {};  // without pairs: exp(-2 pi i b k / N), k = 1 .. N1 - 1
     if constexpr (!L::PFA && SPLIT == 1) {
 #pragma unroll
-        for (int k = 1; k < 4; k++) tw4[k - 1] = static_cast<const C*>(a.zp.tw)[(actA ? ab : 0) * k];
+        for (int k = 1; k < N1; k++) twa[k - 1] = static_cast<const C*>(a.zp.tw)[(actA ? ab : 0) * k];
     }
     // phase-B row
     const int ba = tid % N1, bc = (tid / N1) & 3, bm = tid / (4 * N1);
@@ -140,6 +142,7 @@ __global__ void __launch_bounds__(ZCol<N1, N2, M>::NT, MINB) zcol(const __grid_c
     float4* const row = reinterpret_cast<float4*>(xb + (bm * 4 + bc) * CP + ba * RP);
     // fold: this thread's V neighbouring k_z of columns om, om + OM, ...
     constexpr int V = N % 2 ? 1 : 2, KV = N / V, OM = NT / KV < M ? NT / KV : M, OI = (M + OM - 1) / OM;
+    static_assert(KV <= NT, "a thread for every pair of a column");
     const int om = tid / KV, ok = (tid - om * KV) * V;
     const bool actO = om < OM;
 
@@ -213,10 +216,10 @@ __global__ void __launch_bounds__(ZCol<N1, N2, M>::NT, MINB) zcol(const __grid_c
         for (int at = 0; at < a.nAtom; at++) {
             // ---- phase A
             if ((tid & ~31) < L::IA) {
-                C E[4];
-                float ua[3][4];
+                C E[CA];
+                float ua[3][CA];
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
+                for (int j = 0; j < CA; j++) {
                     const float4 ca = inA[cell0 + j * N2], cb = inB[cell0 + j * N2];
                     const double tu = __hiloint2double(__float_as_int(cb.w), __float_as_int(cb.z));
                     const int ip = inP[cell0 + j * N2] * a.nAtom + at;
@@ -251,17 +254,17 @@ __global__ void __launch_bounds__(ZCol<N1, N2, M>::NT, MINB) zcol(const __grid_c
                 if constexpr (SPLIT == 1) {
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
-                        C v[4];
+                        C v[CA];
 #pragma unroll
-                        for (int j = 0; j < 4; j++) v[j] = q == 0 ? E[j] : make_float2(E[j].x * ua[(q + 2) % 3][j], E[j].y * ua[(q + 2) % 3][j]);
-                        Bfly<4, C>::run(v);
+                        for (int j = 0; j < CA; j++) v[j] = q == 0 ? E[j] : make_float2(E[j].x * ua[(q + 2) % 3][j], E[j].y * ua[(q + 2) % 3][j]);
+                        Bfly<CA, C>::run(v);
                         if constexpr (!L::PFA) {
 #pragma unroll
-                            for (int k = 1; k < 4; k++) v[k] = tw_mul(tw4[k - 1], v[k]);
+                            for (int k = 1; k < CA; k++) v[k] = tw_mul(twa[k - 1], v[k]);
                         }
                         if (actA) {
 #pragma unroll
-                            for (int k = 0; k < 4; k++) st0[q * CP + k * RP] = v[k];
+                            for (int k = 0; k < CA; k++) st0[q * CP + k * RP] = v[k];
                         }
                     }
                 } else {
