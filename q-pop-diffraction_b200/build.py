@@ -26,7 +26,8 @@ LIB = PKG / "libqpopdiff.so"
 OBJ = PKG / "_build"
 
 SOURCES = ["qpd_api.cu", "qpd_noalloc.cu", "qpd_rsm.cu", "qpd_n4000.cu", "qpd_probe.cu", "qpd_any_f32.cu",
-           "qpd_any_f64.cu", "qpd_axisct.cu", "qpd_zcol.cu",
+           "qpd_any_f64.cu", "qpd_axisct.cu", "qpd_axisct_1.cu", "qpd_axisct_2.cu", "qpd_axisct_3.cu",
+           "qpd_axisct_4.cu", "qpd_zcol.cu",
            "qpd_fields.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -766,24 +766,28 @@ template <typename T> struct Impl {
     }
 
     // y or x pass (axis d) on the compile-time register-folding kernels; nfields: fields of the buffer at a.in.
-    // They take every power-of-two length that they have (us, axis_tma -> axis_ct): y pass 1015 -> 745 and x pass
-    // 397 -> 306 at 512x512x104, 3870 -> 2867 and 1577 -> 996 at 1024x1024x68, 167 -> 110 and 74 -> 58 at 256x256x64,
-    // 86 -> 67 and 39 -> 35 at 128^3; the adjoint's x and y passes 395 -> 164 at 256x256x64.
+    // They take every length that they have, 24 to 1024 (N x N x 32: 1.4 to 2.7 times faster than the runtime-length
+    // passes over the list, with odd nz 101 -> 69 for the y pass at 150x135x75; against axis_tma, us: y pass 1015 -> 745 and x pass
+    // 397 -> 306 at 512x512x104, 3870 -> 2285 and 1577 -> 961 at 1024x1024x68, 167 -> 110 and 74 -> 58 at 256x256x64,
+    // 86 -> 60 and 39 -> 31 at 128^3; the adjoint's x and y passes 395 -> 164 at 256x256x64).
     static int ct_axis(qpd_ctx* c, const AxisArgs<T>& a, int d, const AnyFold& f, AnyMode mode, int64_t nfields, int kind,
                        cudaStream_t st, bool* done) {
         *done = false;
         if constexpr (sizeof(T) == 4) {
             const AxisCtShape& s = c->ct[d];
-            // the map's row strides are multiples of 16 bytes for even nz; a launch shape chosen for axis_tma keeps it
+            // a launch shape chosen for axis_tma keeps it
             if (!c->fast || !c->tma || c->knob_oop != 1 || c->knob_nbuf != 2 || (kind >= QPD_K_ADJSEED && !c->knob_adj_tma) ||
-                s.cz == 0 || f.n == 0 || a.nz % 2 != 0 || a.accumulate)
+                s.cz == 0 || f.n == 0 || a.accumulate)
                 return QPD_OK;
             CUtensorMap map;
-            QPD_TRY(field_map(c, &map, const_cast<C*>(a.in), false, a.nz, c->ny, nfields * c->nx, 2 * s.cz,
-                              d == 0 ? 1 : s.box, d == 0 ? s.box : 1));
+            const bool even = a.nz % 2 == 0;  // the map's row strides are multiples of 16 bytes
+            if (!even && !s.odd_nz) return QPD_OK;
+            if (even)
+                QPD_TRY(field_map(c, &map, const_cast<C*>(a.in), false, a.nz, c->ny, nfields * c->nx, 2 * s.cz,
+                                  d == 0 ? 1 : s.box, d == 0 ? s.box : 1));
             cudaEvent_t t0;
             QPD_TRY(tstart(c, st, &t0));
-            QPD_CU(c, launch_axis_ct(map, a, f, static_cast<const C*>(s.stages.tw), mode, d == 0, d == 0 ? c->ny : c->nx, st));
+            QPD_CU(c, launch_axis_ct(even ? &map : nullptr, a, f, static_cast<const C*>(s.stages.tw), mode, d == 0, d == 0 ? c->ny : c->nx, st));
             *done = true;
             return tstop(c, kind, st, t0);
         }
@@ -1718,6 +1722,7 @@ template <typename T> struct Impl {
                         QPD_CU(c, cudaMemcpyAsync(W + g0, h.W, sizeof(T) * cnt, cudaMemcpyHostToDevice, st));
                     } else {  // weights 0 or 1 only: rebuild them from the phase index on the device
                         fill_weight_kernel<T><<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(ph + g0, W + g0, cnt);
+                        c->launches++;
                         QPD_CU(c, cudaGetLastError());
                     }
                 }

@@ -1,4 +1,4 @@
-// Compile-time y and x passes of the float32 fused schedule, the adjoint's included, for power-of-two axes.
+// Compile-time y and x passes of the float32 fused schedule, the adjoint's included.
 //
 // A CTA owns a tile of N rows along the axis by CZ neighbouring z values and walks the pass's input fields; the
 // next field's tile arrives by TMA while the current one is transformed in two or three Stockham stages of radix
@@ -9,10 +9,11 @@
 //
 // Rows hold CZ values, so 16 / CZ rows share the banks of a half-warp; the first stage's outputs of neighbouring
 // threads are R1 rows apart, which would be the same banks: row i of the exchange buffer sits at
-// i ^ ((i / R1) mod (16 / CZ)).  Later stages write neighbouring rows from neighbouring threads.
+// i ^ ((i / R1) mod (16 / CZ)) (odd R1 need none of it).  Later stages write neighbouring rows from neighbouring threads.
 #pragma once
 
 #include "qpd_any.h"
+#include "qpd_axisct.h"
 #include "qpd_fast.cuh"
 #include "qpd_radix.cuh"
 #include "qpd_tma.cuh"
@@ -21,13 +22,13 @@ namespace qpd {
 
 template <int N, int CZ, int NT, int R1, int R2, int R3> struct AxisCt {
     static constexpr int RL = R3 > 1 ? R3 : R2;          // radix of the last stage
-    static constexpr int EPT = N * CZ / NT;              // values per thread
     static constexpr int JT = NT / CZ;                   // butterflies (rows of a stage) done at once
-    static constexpr int TILE = N * CZ;
+    static constexpr int Q1 = cdiv(N / R1, JT), Q2 = cdiv(N / R2, JT), QL = cdiv(N / RL, JT);  // per thread and stage
+    static constexpr int EPT = QL * RL;                  // outputs per thread
+    static constexpr int TILE = (N * CZ + 15) / 16 * 16;
     static constexpr int TW = R1 * any_tw_row(R2) + (R3 > 1 ? R1 * R2 * any_tw_row(R3) : 0);
     static constexpr size_t SMEM = sizeof(float2) * (3 * TILE + TW) + 128;
-    static_assert(R1 * R2 * R3 == N && NT % CZ == 0 && N * CZ % NT == 0, "tile");
-    static_assert(EPT % R1 == 0 && EPT % R2 == 0 && EPT % RL == 0, "whole butterflies per thread");
+    static_assert(R1 * R2 * R3 == N && NT % CZ == 0, "tile");
 };
 
 // v[r] times the twiddle row w (16-byte aligned, values r = 1 ..)
@@ -43,13 +44,19 @@ template <int R> __device__ __forceinline__ void tw_row(float2 (&v)[R], const fl
 template <int N, int CZ, int NT, int R1, int R2, int R3, int MINB, AnyMode MODE, bool XPASS>
 __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUtensorMap map,
                                                     const __grid_constant__ AxisArgs<float> a,
-                                                    const __grid_constant__ AnyFold f, const float2* __restrict__ twg) {
+                                                    const __grid_constant__ AnyFold f, const float2* __restrict__ twg,
+                                                    int tensor) {
     using L = AxisCt<N, CZ, NT, R1, R2, R3>;
     using C = float2;
-    constexpr int EPT = L::EPT, JT = L::JT, TILE = L::TILE, RL = L::RL;
-    constexpr int SW = 16 / CZ > 1 ? 16 / CZ - 1 : 0;
-    constexpr int BOX = tma_rows(N, CZ * (int)sizeof(C));
-    constexpr uint32_t BYTES = TILE * sizeof(C);
+    const bool tma = !ct_odd_nz(N) || tensor;
+    constexpr int EPT = L::EPT, JT = L::JT, TILE = L::TILE, RL = L::RL, QL = L::QL;
+    // rows that share the banks of a half-warp; stage 1's outputs of neighbouring threads meet only when R1 is even
+    constexpr int SW = 16 / CZ > 1 && R1 % (16 / CZ) == 0 ? 16 / CZ - 1 : 0;
+    static_assert(SW == 0 || (JT % (SW + 1) == 0 && N / R2 % R1 == 0 && N / R2 % (SW + 1) == 0), "one swizzle per thread");
+    static_assert(SW == 0 || JT % (R1 * (SW + 1)) == 0 || L::Q2 == 1, "one swizzle per thread");
+    constexpr int BOX = ct_rows(N, CZ * (int)sizeof(C));
+    constexpr uint32_t BYTES = N * CZ * sizeof(C);
+    static_assert(BOX > 0, "a tile is one box, or whole boxes of 128-byte multiples");
     extern __shared__ __align__(128) unsigned char smem_raw[];
     // Three tiles.  Three stages: inputs alternate between tiles 0 and 1, stage 1 writes tile 2, stage 2 writes back
     // into the input's.  Two stages: input i lands in tile i mod 3 and stage 1 writes tile (i + 2) mod 3, since the
@@ -68,6 +75,15 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
         return;
     }
     const int nfx = (int)a.nx;
+    // Input i's tile: one thread's tensor copies, or (odd nz: no tensor map has its row strides) every thread's 8-byte
+    // ones; either completes bar[i & 1].
+    auto issue_threads = [&](int i) {
+        const C* src = a.in + (long long)f.field[i] * a.fstride + (long long)outer * a.ostride + z0 + c;
+        C* dst = tiles + (i % RING) * TILE;
+        if (live)
+            for (int k = j0; k < N; k += JT) cp_async<sizeof(C)>(dst + k * CZ + c, src + k * a.stride);
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bar[i & 1])) : "memory");
+    };
     auto issue = [&](int i) {
         const int b = i & 1, fl = f.field[i];
         C* dst = tiles + (i % RING) * TILE;
@@ -79,13 +95,14 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
         }
     };
     if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        mbar_init(&bar[0], tma ? 1 : NT);
+        mbar_init(&bar[1], tma ? 1 : NT);
         fence_barrier_init();
-        issue(0);
+        if (tma) issue(0);
     }
     for (int i = tid; i < L::TW; i += NT) tw[i] = twg[i];
     __syncthreads();
+    if (!tma) issue_threads(0);
 
     // row offsets of the swizzled stage-1 outputs: s and s ^ (j mod (SW + 1)) differ in the low bits only
     int wofs[SW + 1];
@@ -100,23 +117,26 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
         C* const cur = tiles + (i % RING) * TILE;
         C* const W = tiles + (R3 > 1 ? 2 : (i + 2) % 3) * TILE;
         const C* const cf = static_cast<const C*>(f.coef[i]);
+        // first output row of the thread's butterfly q (row 0 where it has none)
+        auto row_of = [&](int q) { return N / RL % JT == 0 || j0 + q * JT < N / RL ? j0 + q * JT : 0; };
         // with 16 values per thread the fold's coefficients are requested before the input's tile is awaited (1024
         // points: y pass 2850 -> 2290 us at 1024x1024x68); with 8, at 64 registers, they would spill
         constexpr bool EARLY = EPT > 8 && MODE != AnyMode::Pre;
         C cfr[EARLY ? EPT : 1];
         if constexpr (EARLY) {
 #pragma unroll
-            for (int q = 0; q < EPT / RL; q++)
+            for (int q = 0; q < QL; q++)
 #pragma unroll
-                for (int s = 0; s < RL; s++) cfr[q * RL + s] = __ldg(cf + j0 + q * JT + s * (N / RL));
+                for (int s = 0; s < RL; s++) cfr[q * RL + s] = __ldg(cf + row_of(q) + s * (N / RL));
         }
         const bool ok = mbar_wait(&bar[i & 1], (i >> 1) & 1, a.status);
         // ---- stage 1
         {
             constexpr int LR = N / R1;
 #pragma unroll
-            for (int q = 0; q < EPT / R1; q++) {
+            for (int q = 0; q < L::Q1; q++) {
                 const int j = j0 + q * JT;  // j mod (SW + 1) = j0 mod (SW + 1)
+                if (LR % JT != 0 && j >= LR) break;
                 C v[R1];
 #pragma unroll
                 for (int r = 0; r < R1; r++) v[r] = cur[(j + r * LR) * CZ + c];
@@ -133,18 +153,24 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
         if (!__syncthreads_and(ok)) return;  // a load never landed; no other is in flight
         // the next input's tile: its last readers (three stages: stage 3, two: stage 2 of the input before) are past
         // this barrier
-        if (tid == 0 && i + 1 < f.n) {
+        if (!tma) {
+            if (i + 1 < f.n) issue_threads(i + 1);
+        } else if (tid == 0 && i + 1 < f.n) {
             fence_proxy_async();
             issue(i + 1);
         }
         // ---- stage 2
         C x[EPT];
+        if constexpr (L::QL * JT != N / RL) {
+#pragma unroll
+            for (int e = 0; e < EPT; e++) x[e] = make_float2(0.f, 0.f);
+        }
         {
             constexpr int LR = N / R2;
-            static_assert(JT % (R1 * (SW + 1)) == 0 || EPT == R2, "the swizzle of a thread's rows is one constant");
 #pragma unroll
-            for (int q = 0; q < EPT / R2; q++) {
+            for (int q = 0; q < L::Q2; q++) {
                 const int j = j0 + q * JT;
+                if (LR % JT != 0 && j >= LR) break;
                 C v[R2];
 #pragma unroll
                 for (int r = 0; r < R2; r++) {
@@ -170,8 +196,9 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
             __syncthreads();
             constexpr int LR = N / R3;
 #pragma unroll
-            for (int q = 0; q < EPT / R3; q++) {
+            for (int q = 0; q < QL; q++) {
                 const int j = j0 + q * JT;
+                if (LR % JT != 0 && j >= LR) break;
                 C v[R3];
 #pragma unroll
                 for (int r = 0; r < R3; r++) v[r] = cur[(j + r * LR) * CZ + c];
@@ -181,14 +208,17 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
                 for (int s = 0; s < R3; s++) x[q * R3 + s] = v[s];
             }
         }
+        // a thread without a butterfly at q folds zeros with the coefficients of row 0
+        constexpr int LL = N / RL;
+        auto has = [&](int q) { return LL % JT == 0 || j0 + q * JT < LL; };
         // ---- fold: x[q RL + s] is output row k = j0 + q JT + s N / RL
 #pragma unroll
-        for (int q = 0; q < EPT / RL; q++)
+        for (int q = 0; q < QL; q++)
 #pragma unroll
             for (int s = 0; s < RL; s++) {
                 const int e = q * RL + s;
                 if constexpr (MODE == AnyMode::Pre) acc[e] = x[e];
-                else fold_fma(acc[e], EARLY ? cfr[EARLY ? e : 0] : __ldg(cf + j0 + q * JT + s * (N / RL)), x[e]);
+                else fold_fma(acc[e], EARLY ? cfr[EARLY ? e : 0] : __ldg(cf + row_of(q) + s * (N / RL)), x[e]);
             }
         if (!f.last[i]) continue;
         if (live) {
@@ -196,9 +226,10 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
             if constexpr (MODE == AnyMode::Store || MODE == AnyMode::Pre) {
                 C* const dst = a.out + (long long)f.out[i] * a.fstride + base;
 #pragma unroll
-                for (int q = 0; q < EPT / RL; q++)
+                for (int q = 0; q < QL; q++)
 #pragma unroll
-                    for (int s = 0; s < RL; s++) dst[(j0 + q * JT + s * (N / RL)) * a.stride] = acc[q * RL + s];
+                    for (int s = 0; s < RL; s++)
+                        if (has(q)) dst[(j0 + q * JT + s * (N / RL)) * a.stride] = acc[q * RL + s];
             } else {
                 const int ky = outer, kz = z0 + c, ny = (int)a.ny;
                 const int sy = fftshift_at(ky, ny), sz = fftshift_at(kz, a.nz);
@@ -207,21 +238,22 @@ __global__ void __launch_bounds__(NT, MINB) axis_ct(const __grid_constant__ CUte
                 double gi[MODE == AnyMode::Seed ? EPT : 1];
                 if constexpr (MODE == AnyMode::Seed) {  // all in flight before the first is needed
 #pragma unroll
-                    for (int q = 0; q < EPT / RL; q++)
+                    for (int q = 0; q < QL; q++)
 #pragma unroll
                         for (int s = 0; s < RL; s++) {
                             const int k = j0 + q * JT + s * (N / RL);
-                            gi[q * RL + s] = __ldg(a.gI + ((long long)(k < N / 2 ? k + N / 2 : k - N / 2) * ny + sy) * a.nz + sz);
+                            gi[q * RL + s] = has(q) ? __ldg(a.gI + ((long long)fftshift_at(k, N) * ny + sy) * a.nz + sz) : 0.0;
                         }
                 }
 #pragma unroll
-                for (int q = 0; q < EPT / RL; q++)
+                for (int q = 0; q < QL; q++)
 #pragma unroll
                     for (int s = 0; s < RL; s++) {
                         const int k = j0 + q * JT + s * (N / RL), e = q * RL + s;
+                        if (!has(q)) continue;
                         const double S = a.S[0][k] * syz;
                         const double re = (double)acc[e].x, im = (double)acc[e].y;
-                        const long long at = ((long long)(k < N / 2 ? k + N / 2 : k - N / 2) * ny + sy) * a.nz + sz;
+                        const long long at = ((long long)fftshift_at(k, N) * ny + sy) * a.nz + sz;
                         if constexpr (MODE == AnyMode::Intensity) {
                             a.I[at] = floor_1e50(S * S * (re * re + im * im) * a.scale2);
                         } else {

@@ -1,0 +1,6 @@
+// Part 2 of the compile-time y and x passes.
+#include "qpd_axisct_part.cuh"
+
+namespace qpd {
+QPD_AXIS_CT_PART(launch_axis_ct_2, QPD_AXIS_CT_2)
+}  // namespace qpd
