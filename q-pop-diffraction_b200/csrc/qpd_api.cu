@@ -1706,8 +1706,9 @@ template <typename T> struct Impl {
                 });
                 const uint32_t f = fl.load();
                 flags |= f;
-                // the 3 planes of P and the 3 of U follow one another on both sides
-                if (sizeof(T) * (size_t)n <= (size_t)0x7fffffff) {  // a 2-D copy's pitch is at most 2^31 - 1 bytes
+                // the 3 planes of P and the 3 of U follow one another on both sides: one 2-D copy for the small chunks of
+                // pageable arrays (its pitch is at most 2^31 - 1 bytes), six plain ones for the large ones
+                if (paged && sizeof(T) * (size_t)n <= (size_t)0x7fffffff) {
                     QPD_CU(c, cudaMemcpy2DAsync(P + g0, sizeof(T) * n, h.P, sizeof(T) * C, sizeof(T) * cnt, 6, cudaMemcpyHostToDevice, st));
                 } else {
                     for (int k = 0; k < 6; k++)
