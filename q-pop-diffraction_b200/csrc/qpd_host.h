@@ -13,6 +13,7 @@
 #include <condition_variable>
 #include <cstdint>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -20,6 +21,9 @@
 namespace qpd {
 
 // A fixed set of threads running one parallel-for at a time.
+//
+// Every job is an object of its own, with its own indices and its own count of unfinished ones: a worker that is late
+// out of one job still holds that job, whose indices are used up, and cannot take or count an index of the next.
 class Workers {
    public:
     explicit Workers(int n) {
@@ -38,50 +42,52 @@ class Workers {
     // f(i) for i in [0, count), spread over the workers and the calling thread; returns when done.
     void parallel(int count, const std::function<void(int)>& f) {
         if (count <= 0) return;
+        const auto job = std::make_shared<Job>(f, count);
         {
             std::lock_guard<std::mutex> g(m_);
-            job_ = &f;
-            count_ = count;
-            next_.store(0);
-            left_ = count;
-            gen_++;
+            job_ = job;
         }
         cv_.notify_all();
-        work();
+        work(*job);
         std::unique_lock<std::mutex> g(m_);
-        done_.wait(g, [this] { return left_ == 0; });
-        job_ = nullptr;
+        done_.wait(g, [&] { return job->left.load() == 0; });
+        job_.reset();
     }
 
    private:
-    void work() {
+    struct Job {
+        const std::function<void(int)>& f;  // alive while left > 0: called for indices below count only
+        const int count;
+        std::atomic<int> next{0}, left;
+        Job(const std::function<void(int)>& fn, int n) : f(fn), count(n), left(n) {}
+    };
+    void work(Job& job) {
         for (;;) {
-            const int i = next_.fetch_add(1);
-            if (i >= count_) return;
-            (*job_)(i);
-            std::lock_guard<std::mutex> g(m_);
-            if (--left_ == 0) done_.notify_all();
+            const int i = job.next.fetch_add(1);
+            if (i >= job.count) return;
+            job.f(i);
+            if (job.left.fetch_sub(1) == 1) {
+                std::lock_guard<std::mutex> g(m_);  // the caller is waiting, or has yet to look at `left`
+                done_.notify_all();
+            }
         }
     }
     void loop() {
-        uint64_t seen = 0;
+        std::shared_ptr<Job> job;  // the last one worked on, kept so that its address is not used again meanwhile
         for (;;) {
             {
                 std::unique_lock<std::mutex> g(m_);
-                cv_.wait(g, [&] { return stop_ || (gen_ != seen && job_ != nullptr); });
+                cv_.wait(g, [&] { return stop_ || (job_ && job_ != job); });
                 if (stop_) return;
-                seen = gen_;
+                job = job_;
             }
-            work();
+            work(*job);
         }
     }
     std::vector<std::thread> th_;
     std::mutex m_;
     std::condition_variable cv_, done_;
-    const std::function<void(int)>* job_ = nullptr;
-    std::atomic<int> next_{0};
-    int count_ = 0, left_ = 0;
-    uint64_t gen_ = 0;
+    std::shared_ptr<Job> job_;  // the job that workers join (under m_)
     bool stop_ = false;
 };
 
