@@ -21,6 +21,7 @@
 
 #include "qpd_any.h"
 #include "qpd_radix.cuh"
+#include "qpd_smem.h"
 #include "qpd_tma.cuh"
 
 namespace qpd {
@@ -476,14 +477,9 @@ inline AnyDev any_dev(const AnyStages& st, int lp) {
     return d;
 }
 
-template <typename K> cudaError_t any_smem_attr(K k, size_t bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 template <typename T, AnyMode MODE>
 cudaError_t launch_axis_mode(const AxisAny<T>& g, int ept, unsigned grid, int nt, size_t smem, cudaStream_t st) {
-    cudaError_t e = ept == 8 ? any_smem_attr(axis_any<T, 8, MODE>, smem) : any_smem_attr(axis_any<T, 16, MODE>, smem);
+    cudaError_t e = ept == 8 ? allow_smem<axis_any<T, 8, MODE>>(smem) : allow_smem<axis_any<T, 16, MODE>>(smem);
     if (e != cudaSuccess) return e;
     if (ept == 8) axis_any<T, 8, MODE><<<grid, nt, smem, st>>>(g);
     else axis_any<T, 16, MODE><<<grid, nt, smem, st>>>(g);
@@ -578,7 +574,7 @@ cudaError_t launch_z_any(const ZArgs<T>& a, const AnyStages& st, int sms, size_t
     *done = z_tile(a, st, sms, smem_max, &t);
     if (!*done) return cudaSuccess;
     const AnyDev d = any_dev(st, t.lm + 2);
-    cudaError_t e = t.cpt == 2 ? any_smem_attr(zstage_any<T, 2>, t.smem) : any_smem_attr(zstage_any<T, 4>, t.smem);
+    cudaError_t e = t.cpt == 2 ? allow_smem<zstage_any<T, 2>>(t.smem) : allow_smem<zstage_any<T, 4>>(t.smem);
     if (e != cudaSuccess) return e;
     if (t.cpt == 2) zstage_any<T, 2><<<(unsigned)t.grid, t.nt, t.smem, stream>>>(a, d, z_magic(a.nz));
     else zstage_any<T, 4><<<(unsigned)t.grid, t.nt, t.smem, stream>>>(a, d, z_magic(a.nz));
@@ -592,7 +588,7 @@ cudaError_t launch_adjz_any(const AdjZArgs<T>& a, const AnyStages& st, int sms, 
     *done = z_tile(a.z, st, sms, smem_max, &t);
     if (!*done) return cudaSuccess;
     const AnyDev d = any_dev(st, t.lm + 2);
-    cudaError_t e = t.cpt == 2 ? any_smem_attr(adj_zstage_any<T, 2>, t.smem) : any_smem_attr(adj_zstage_any<T, 4>, t.smem);
+    cudaError_t e = t.cpt == 2 ? allow_smem<adj_zstage_any<T, 2>>(t.smem) : allow_smem<adj_zstage_any<T, 4>>(t.smem);
     if (e != cudaSuccess) return e;
     if (t.cpt == 2) adj_zstage_any<T, 2><<<(unsigned)t.grid, t.nt, t.smem, stream>>>(a, d, z_magic(a.z.nz));
     else adj_zstage_any<T, 4><<<(unsigned)t.grid, t.nt, t.smem, stream>>>(a, d, z_magic(a.z.nz));

@@ -26,6 +26,7 @@
 #include "qpd_host.h"
 #include "qpd_kernels.cuh"
 #include "qpd_n4000.h"
+#include "qpd_smem.h"
 
 namespace qpd {
 // qpd_probe.cu: a kernel that takes the bounded-wait failure path (a barrier no copy completes)
@@ -318,9 +319,8 @@ size_t max_smem(qpd_ctx* c) {
     return (size_t)v;
 }
 
-template <typename K> int set_smem(qpd_ctx* c, K kernel, size_t bytes) {
-    if (bytes > 48 * 1024)
-        QPD_CU(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+template <auto K> int set_smem(qpd_ctx* c, size_t bytes) {
+    QPD_CU(c, allow_smem<K>(bytes));
     return QPD_OK;
 }
 
@@ -701,7 +701,7 @@ template <typename T> struct Impl {
         a.M = std::max(1, (int)std::min<int64_t>(cap / a.nz, a.ncols));
         a.ps = odd_stride(a.nz);
         const size_t smem = sizeof(C) * 4 * a.M * a.ps + sizeof(AtomPhase<T>) * a.in.nPhase * a.nAtom + 16;
-        QPD_TRY(set_smem(c, zstage_kernel<T, NT, EPT>, smem));
+        QPD_TRY((set_smem<zstage_kernel<T, NT, EPT>>(c, smem)));
         const int64_t grid = (a.ncols + a.M - 1) / a.M;
         cudaEvent_t t0;
         QPD_TRY(tstart(c, st, &t0));
@@ -729,7 +729,7 @@ template <typename T> struct Impl {
         a.M = std::max(1, (int)std::min<int64_t>(NT * EPT / a.nz, a.ncols));
         a.ps = odd_stride(a.nz);
         const size_t smem = sizeof(C) * a.M * a.ps + 16;
-        QPD_TRY(set_smem(c, fftz_kernel<T, NT, EPT>, smem));
+        QPD_TRY((set_smem<fftz_kernel<T, NT, EPT>>(c, smem)));
         const int64_t grid = (a.ncols + a.M - 1) / a.M;
         cudaEvent_t t0;
         QPD_TRY(tstart(c, st, &t0));
@@ -757,7 +757,7 @@ template <typename T> struct Impl {
         a.Cz = std::max(1, std::min(a.nz, NT * EPT / a.N));
         a.nzc = (a.nz + a.Cz - 1) / a.Cz;
         const size_t smem = sizeof(C) * a.N * a.Cz + 16;
-        QPD_TRY(set_smem(c, axis_kernel<T, NT, EPT, EPI>, smem));
+        QPD_TRY((set_smem<axis_kernel<T, NT, EPT, EPI>>(c, smem)));
         const int64_t grid = nouter * a.nzc;
         cudaEvent_t t0;
         QPD_TRY(tstart(c, st, &t0));
@@ -842,7 +842,7 @@ template <typename T> struct Impl {
         a.Cz = std::max(1, std::min(a.nz, NT * EPT / a.N));
         a.nzc = (a.nz + a.Cz - 1) / a.Cz;
         const size_t smem = sizeof(C) * a.N * a.Cz + 16;
-        QPD_TRY(set_smem(c, adj_axis_kernel<T, NT, EPT>, smem));
+        QPD_TRY((set_smem<adj_axis_kernel<T, NT, EPT>>(c, smem)));
         cudaEvent_t t0;
         QPD_TRY(tstart(c, st, &t0));
         adj_axis_kernel<T, NT, EPT><<<(unsigned)(nouter * a.nzc), NT, smem, st>>>(a);
@@ -900,7 +900,7 @@ template <typename T> struct Impl {
         a.z.M = std::max(1, (int)std::min<int64_t>(cap / a.z.nz, a.z.ncols));
         a.z.ps = odd_stride(a.z.nz);
         const size_t smem = sizeof(C) * 4 * a.z.M * a.z.ps + sizeof(AtomPhase<T>) * a.z.in.nPhase * a.z.nAtom + 16;
-        QPD_TRY(set_smem(c, adj_zstage_kernel<T, NT, EPT>, smem));
+        QPD_TRY((set_smem<adj_zstage_kernel<T, NT, EPT>>(c, smem)));
         const int64_t grid = (a.z.ncols + a.z.M - 1) / a.z.M;
         cudaEvent_t t0;
         QPD_TRY(tstart(c, st, &t0));
@@ -915,7 +915,7 @@ template <typename T> struct Impl {
         // transform buffer (4 planes), two stages of the 3 input fields, the atom table
         const size_t smem = sizeof(C) * (4 * M * PS + 6 * M * NZ) + sizeof(AtomPhase<T>) * a.z.in.nPhase * a.z.nAtom + 16;
         if (smem > max_smem(c)) return run_adj_z(c, a, st);
-        QPD_TRY(set_smem(c, adj_zstage_fast<T, NZ, M, NT, RAD>, smem));
+        QPD_TRY((set_smem<adj_zstage_fast<T, NZ, M, NT, RAD>>(c, smem)));
         const int64_t grid = (a.z.ncols + M - 1) / M;
         cudaEvent_t t0;
         QPD_TRY(tstart(c, st, &t0));
@@ -945,7 +945,7 @@ template <typename T> struct Impl {
         a.M = M;
         a.ps = PS;
         const size_t smem = sizeof(C) * 4 * M * PS + sizeof(AtomPhase<T>) * a.in.nPhase * a.nAtom + 16;
-        QPD_TRY(set_smem(c, zstage_fast<T, NZ, M, NT, RAD>, smem));
+        QPD_TRY((set_smem<zstage_fast<T, NZ, M, NT, RAD>>(c, smem)));
         const int64_t grid = (a.ncols + M - 1) / M;
         cudaEvent_t t0;
         QPD_TRY(tstart(c, st, &t0));
@@ -969,7 +969,7 @@ template <typename T> struct Impl {
         a.ps = L::PS;
         const size_t smem = L::bytes(a.in.nPhase * a.nAtom, a.nAtom);
         if (smem > max_smem(c)) return fail(c, QPD_ERR_UNSUPPORTED, "z stage tables exceed shared memory");
-        QPD_TRY(set_smem(c, zstage_pipe<T, NZ, M, NT, RAD, REGIN>, smem));
+        QPD_TRY((set_smem<zstage_pipe<T, NZ, M, NT, RAD, REGIN>>(c, smem)));
         int per_sm = 0, sms = 0;
         QPD_CU(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, zstage_pipe<T, NZ, M, NT, RAD, REGIN>, NT,
                                                                 smem));
@@ -989,7 +989,7 @@ template <typename T> struct Impl {
         a.ps = L::PS;
         const size_t smem = L::bytes(a.in.nPhase * a.nAtom, a.nAtom);
         if (smem > max_smem(c)) return fail(c, QPD_ERR_UNSUPPORTED, "z stage tables exceed shared memory");
-        QPD_TRY(set_smem(c, zstage_pfa<T, N1, N2>, smem));
+        QPD_TRY((set_smem<zstage_pfa<T, N1, N2>>(c, smem)));
         int per_sm = 0, sms = 0;
         QPD_CU(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, zstage_pfa<T, N1, N2>, NT, smem));
         QPD_CU(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
@@ -1062,7 +1062,7 @@ template <typename T> struct Impl {
         a.Cz = CZ;
         a.nzc = (a.nz + CZ - 1) / CZ;
         const size_t smem = sizeof(C) * N * CZ + 16;
-        QPD_TRY(set_smem(c, axis_fast<T, N, CZ, NT, VEC, EPI, RAD>, smem));
+        QPD_TRY((set_smem<axis_fast<T, N, CZ, NT, VEC, EPI, RAD>>(c, smem)));
         const int64_t grid = nouter * a.nzc;
         cudaEvent_t t0;
         QPD_TRY(tstart(c, st, &t0));
@@ -1095,7 +1095,7 @@ template <typename T> struct Impl {
                           2 * CZ, XP ? 1 : BOX, XP ? BOX : 1));
         const size_t smem = sizeof(C) * N * CZ * (NBUF + (OOP ? 1 : 0)) + sizeof(C) * N + 128;
         if (smem > max_smem(c)) return fail(c, QPD_ERR_UNSUPPORTED, "axis tile exceeds shared memory");
-        QPD_TRY(set_smem(c, axis_tma<T, N, CZ, NT, VEC, EPI, XP, RAD, NBUF, OOP, YZ, PRE, SEED>, smem));
+        QPD_TRY((set_smem<axis_tma<T, N, CZ, NT, VEC, EPI, XP, RAD, NBUF, OOP, YZ, PRE, SEED>>(c, smem)));
         const int64_t grid = nouter * a.nzc;
         cudaEvent_t t0;
         QPD_TRY(tstart(c, st, &t0));
@@ -1107,7 +1107,7 @@ template <typename T> struct Impl {
     template <int N, int NT, class RAD> static int bulk_axis_(qpd_ctx* c, AxisArgs<T>& a, cudaStream_t st) {
         const size_t smem = sizeof(C) * (3 * N + (N + 63) / 64 + 64) + 128;
         if (smem > max_smem(c)) return fail(c, QPD_ERR_UNSUPPORTED, "axis pencils exceed shared memory");
-        QPD_TRY(set_smem(c, axis_bulk<T, N, NT, RAD>, smem));
+        QPD_TRY((set_smem<axis_bulk<T, N, NT, RAD>>(c, smem)));
         const int64_t grid = c->nx * c->nz;
         cudaEvent_t t0;
         QPD_TRY(tstart(c, st, &t0));

@@ -4,6 +4,7 @@
 #include "qpd_axisct.cuh"
 #include "qpd_axisct.h"
 #include "qpd_axisct_lengths.h"
+#include "qpd_smem.h"
 
 namespace qpd {
 namespace {
@@ -17,7 +18,7 @@ cudaError_t go(const CUtensorMap* map, AxisArgs<float> a, const AnyFold& f, cons
     a.nzc = (a.nz + CZ - 1) / CZ;
     const long long grid = nouter * a.nzc;
     if ((!map && !ct_odd_nz(N)) || grid < 1 || grid > 0x7fffffffLL || f.n < 1) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM);
+    cudaError_t e = allow_smem<axis_ct<N, CZ, NT, R1, R2, R3, MINB, MODE, XPASS>>(L::SMEM);
     if (e != cudaSuccess) return e;
     k<<<(unsigned)grid, NT, L::SMEM, st>>>(map ? *map : CUtensorMap{}, a, f, tw, map != nullptr);
     return cudaGetLastError();

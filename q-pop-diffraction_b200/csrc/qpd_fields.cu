@@ -1,6 +1,8 @@
 // Kernel and launch of the boundary-input preparation (qpd_fields.h).
 #include "qpd_fields.h"
 
+#include "qpd_smem.h"
+
 namespace qpd {
 
 // Dynamic shared memory: ramp (double) + phase index (char) + one float tile per input plane.
@@ -155,7 +157,7 @@ template <typename T> __global__ void __launch_bounds__(kFT * kFRows) fields_ker
 template <typename T> cudaError_t launch_fields(const FieldsArgs<T>& a, cudaStream_t st) {
     const int planes = a.nStruc + (a.u[0] ? 3 : 0) + (a.phase ? a.nPhase : 0) + (a.region ? 1 : 0);
     const size_t smem = fields_smem_bytes(planes);
-    cudaError_t e = cudaFuncSetAttribute(fields_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<fields_kernel<T>>(smem);
     if (e != cudaSuccess) return e;
     const long long cols = (a.nx * a.ny + kFT - 1) / kFT, chunks = (a.z0 + a.nz + kFT - 1) / kFT - a.z0 / kFT;
     if (cols > 0x7fffffffLL || chunks > 65535) return cudaErrorInvalidValue;

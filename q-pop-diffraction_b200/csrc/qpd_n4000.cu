@@ -21,6 +21,7 @@
 // staging buffer while the current one is transformed, completing on an mbarrier whose waits are
 // bounded (a copy that never lands records QPD_DEVERR_TIMEOUT in the status word and ends the CTA).
 #include "qpd_n4000.h"
+#include "qpd_smem.h"
 #include "qpd_tma.cuh"
 
 namespace qpd {
@@ -527,7 +528,7 @@ cudaError_t launch_strided(const CUtensorMap& map, const AxisArgs<float>& a, con
     if (a.N != kN || a.nx < 1 || a.nz % 2 != 0 || nouter < 1 || p.n < 1 || p.n > kPass4kMax)
         return cudaErrorInvalidValue;
     const size_t smem = sizeof(float2) * (kTile + 2 * kPen + kTW + 20 * p.n);
-    cudaError_t e = cudaFuncSetAttribute(strided4000<EPI, YZ, MID>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<strided4000<EPI, YZ, MID>>(smem);
     if (e != cudaSuccess) return e;
     const long long ntiles = (long long)nouter * (a.nz / 2);
     if (ntiles + sm_count() >= (1LL << 31)) return cudaErrorInvalidValue;  // tiles index in 32 bits
@@ -543,7 +544,7 @@ cudaError_t launch_unstage_intensity(const double* T, double* I, long long nx, l
     const long long ntiles = ny * ((nx + kUX - 1) / kUX);
     if (nx < 1 || ny < 1 || nz < 1 || nz > 256 || ntiles >= (1LL << 31)) return cudaErrorInvalidValue;
     const size_t smem = sizeof(double) * kUP * nz;
-    cudaError_t e = cudaFuncSetAttribute(unstage_intensity, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<unstage_intensity>(smem);
     if (e != cudaSuccess) return e;
     const long long grid = std::min<long long>(ntiles, 4LL * sm_count());
     unstage_intensity<<<(unsigned)grid, kUT, smem, st>>>(T, I, (int)nx, (int)ny, (int)nz, (int)ntiles);
@@ -553,7 +554,7 @@ cudaError_t launch_unstage_intensity(const double* T, double* I, long long nx, l
 cudaError_t launch_ypass4000(const AxisArgs<float>& a, const Pass4k& p, long long npencils, cudaStream_t st) {
     if (p.n < 1 || p.n > kPass4kMax || npencils < 1) return cudaErrorInvalidValue;
     const size_t smem = sizeof(float2) * (kN + kSA + kSB + kTW + 20 * p.n);
-    cudaError_t e = cudaFuncSetAttribute(ypass4000, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<ypass4000>(smem);
     if (e != cudaSuccess) return e;
     const long long grid = std::min<long long>(npencils, 2LL * sm_count());
     ypass4000<<<(unsigned)grid, kT, smem, st>>>(a, p, npencils);

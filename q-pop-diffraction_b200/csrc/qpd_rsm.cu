@@ -18,6 +18,7 @@
 #include <string>
 
 #include "qpopdiff.h"
+#include "qpd_smem.h"
 
 void qpd_internal_set_error(const char* msg);
 
@@ -86,7 +87,7 @@ int qpd_rsm_project(const double* I, int64_t nx, int64_t ny, int64_t nz, double*
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (xy || xz) {
         const size_t smem = sizeof(double) * (size_t)ny;
-        cudaError_t e = cudaFuncSetAttribute(rsm_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = qpd::allow_smem<rsm_x_kernel>(smem);
         if (e != cudaSuccess) return fail(std::string("qpd_rsm_project: ") + cudaGetErrorString(e), QPD_ERR_CUDA);
         rsm_x_kernel<<<(unsigned)nx, dim3(kRT, kRRows), smem, st>>>(I, ny, nz, xy, xz);
         e = cudaGetLastError();

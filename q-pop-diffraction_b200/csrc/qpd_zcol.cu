@@ -1,6 +1,7 @@
 // Instantiations and launch of the float32 z stage (qpd_zcol.cuh).
 #include <algorithm>
 
+#include "qpd_smem.h"
 #include "qpd_zcol.cuh"
 #include "qpd_zcol.h"
 
@@ -14,7 +15,7 @@ cudaError_t go(const ZArgs<float>& a, int cta_tiles, int sms, size_t smem_max, c
     *done = smem <= smem_max;
     if (!*done) return cudaSuccess;
     auto k = zcol<N1, N2, M, MINB, ISO>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<zcol<N1, N2, M, MINB, ISO>>(smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, L::NT, smem);
