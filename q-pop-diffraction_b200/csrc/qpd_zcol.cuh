@@ -25,6 +25,7 @@
 
 #include "qpd_kernels.cuh"
 #include "qpd_radix.cuh"
+#include "qpd_zprefetch.h"
 
 namespace qpd {
 
@@ -157,13 +158,13 @@ __global__ void __launch_bounds__(ZCol<N1, N2, M>::NT, MINB) zcol(const __grid_c
         // the next tile's inputs come closer while this one is computed
         const long long gn = (t + gridDim.x) * CELLS;
         if (gn + CELLS <= a.ncols * N) {
-            constexpr int LINES = (CELLS * 4 + 127) / 128;
-            for (int i = tid; i < 7 * LINES; i += NT) {
-                const int k = i / LINES, l = i - k * LINES;
-                const void* q = k < 3 ? (const void*)(a.in.P + k * a.in.n + gn + 32 * l)
-                              : k < 6 ? (const void*)(a.in.U + (k - 3) * a.in.n + gn + 32 * l)
-                                      : (const void*)(a.in.phase + gn + 32 * l);
-                if (k < 6 || l % 4 == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
+            const int nl = prefetch_lines(CELLS, a.in.nStruc);
+            for (int i = tid; i < nl; i += NT) {
+                const PrefetchLine l = prefetch_line(i, CELLS, a.in.nStruc, a.in.n, gn);
+                const void* q = l.array == 0 ? (const void*)(a.in.P + l.at)
+                              : l.array == 1 ? (const void*)(a.in.U + l.at)
+                                             : (const void*)(a.in.phase + l.at);
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
             }
         }
         // ---- inputs, neighbouring threads on neighbouring z
