@@ -1602,10 +1602,14 @@ template <typename T> struct Impl {
         }
         for (auto& e : c->ring_ev)
             if (!e) QPD_CU(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        // Pageable arrays (NumPy's) cross a device copy through the driver's own staging, one thread at about
-        // 10 GB/s, where the workers read them at several times that and the packed chunk is pinned: every chunk is
-        // packed on the host then, in at least 4 chunks so that the copies overlap the packing (a 96x96x64 call took 4.7 ms the driver's way and
-        // takes 1.1 ms, with the result coming back through the ring below).
+        // Pageable arrays (NumPy's) cross a device copy through the driver's own staging, one thread at about 10 GB/s,
+        // where the workers read them at several times that and the packed chunk is pinned.  With a worker beside the
+        // calling thread, every chunk is packed on the host then, in at least 4 chunks so that the copies overlap the
+        // packing, and the result comes back through the ring below.  ms per call, two routes -> here, at 16, 4 and 2
+        // packing threads: 2.6 -> 1.1, 2.7 -> 1.3 and 2.7 -> 2.0 at 96x96x64; 14.7 -> 3.8, 14.7 -> 5.1 and 14.0 -> 8.7
+        // at 128^3; 51 -> 35, 77 -> 72 and 119 -> 117 at 512x512x104; 107 -> 78 and 179 -> 162 (4 threads) at
+        // 1024x1024x68.  A calling thread that packs alone is slower than the driver (2.8 -> 3.8 at 96x96x64, 209 -> 222
+        // at 512x512x104): it keeps the two routes.
         auto pageable = [](const void* p) {
             cudaPointerAttributes at;
             if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -1614,7 +1618,8 @@ template <typename T> struct Impl {
             }
             return at.type == cudaMemoryTypeUnregistered;
         };
-        const bool paged = pageable(oPhase) || pageable(u) || (NS > 0 && pageable(oStruc)) || (region && pageable(region));
+        const bool helped = c->workers->size() > 0;
+        const bool paged = helped && (pageable(oPhase) || pageable(u) || (NS > 0 && pageable(oStruc)) || (region && pageable(region)));
         int64_t C = std::min<int64_t>(n, (int64_t)1 << 21);  // cells per chunk
         if (paged) C = std::min<int64_t>(C, std::max<int64_t>((int64_t)1 << 16, ((n + 3) / 4 + 63) / 64 * 64));
         constexpr int NSLOT = 3;
@@ -1752,7 +1757,7 @@ template <typename T> struct Impl {
         double* Id = static_cast<double*>(c->Idev.p);
         QPD_TRY(run_device(c, in, Id, st));
         const size_t total = sizeof(double) * n;
-        if (!pageable(I) || c->hring_bytes < NSLOT * (size_t)4096) {
+        if (!helped || !pageable(I) || c->hring_bytes < NSLOT * (size_t)4096) {
             QPD_CU(c, cudaMemcpyAsync(I, Id, total, cudaMemcpyDeviceToHost, st));
             QPD_CU(c, cudaStreamSynchronize(st));
         } else {
