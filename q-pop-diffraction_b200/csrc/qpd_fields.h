@@ -7,14 +7,15 @@
 // phases of the FE materials, region = (cell is FE) x region file, and the u_z reference ramp
 // (cumsum_z dc[mat] - dc[mat] / 2) dz summed over the FULL material stack, then cropped.
 //
-// Layout: a block owns 32 neighbouring columns of the (y, x) plane, in file order, and one chunk of 32
-// layers.  Its planes are read with the columns fastest (coalesced in the file order) by warps 1..7 while
-// warp 0 runs each column's ramp serially in float64 from layer 0 up to the chunk, in the order of
-// numpy.cumsum (a block repeats the sums of the chunks below it, 1 byte per layer and column, so that
-// chunks need not wait for one another); the cropped layers are written transposed with z fastest
-// (coalesced in the kernel order) through padded shared tiles.  Bound by memory traffic on volumes and
-// by the serial sum on films: 1x400x400 takes 24 us on 13 x 13 blocks, where blocks of one y row and 32 x
-// that walked the chunks in turn, reading a plane at a time, took 95 us.
+// Layout: a block owns 32 neighbouring columns of the (y, x) plane, in file order, and one or more chunks of 32 layers
+// (qpd_fields_split.h).  A chunk's planes are read with the columns fastest (coalesced in the file order) by warps 1..7
+// while warp 0 runs each column's ramp serially in float64, in the order of numpy.cumsum, from layer 0 up to the block's
+// first chunk and then through its chunks (1 byte per layer and column); the cropped layers are written transposed with z
+// fastest (coalesced in the kernel order) through padded shared tiles.  Bound by memory traffic on volumes and by the
+// serial sum on films, so a film's chunks have blocks of their own, which repeat the sums of the layers below, and a wide
+// plane's columns sum every layer once.  us per kernel, blocks that walk all chunks of 32 x in one y row, a plane at a
+// time -> a block per chunk -> here: 1x400x400 97 -> 24 -> 24, 256x256x64 111 -> 82 -> 82, 512x512x104 637 -> 658 -> 629,
+// 1024x1024x68 1810 -> 2373 -> 1809, 256x256x1024 1614 -> 3278 -> 1340, 512x512x104 from layer 500 1338 -> 2018 -> 885.
 #pragma once
 
 #include "qpd_kernels.cuh"
@@ -45,6 +46,7 @@ template <typename T> struct FieldsArgs {
 
 constexpr int kFT = 32;        // tile edge (x and z)
 constexpr int kFRows = 8;      // threadIdx.y extent
+constexpr int kFieldsBlocks = 12 * 148;  // blocks that fill the device: three rounds of four per SM (6 and 8 per SM: 128^3 49 -> 52 us)
 constexpr int kFPitch = kFT + 1;
 
 template <typename T> cudaError_t launch_fields(const FieldsArgs<T>& a, cudaStream_t st);
