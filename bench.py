@@ -32,8 +32,8 @@ Printed (rank 0, one JSON line):
             end-to-end volume from float64 host arrays through qpd_run_host).
 
 With --impl reference only the reference's own diffraction() runs (rank 0, NumPy with its own
-threading, as the reference computes), on a bounded crop of the workload per step; the oracle
-port stands in when baseline/_ref is absent.
+threading, as the reference computes), on a bounded crop of the workload per step; with neither
+baseline/_ref nor a source checkout there is nothing to run, and the line says so.
 Under torchrun each rank evaluates its own volumes on its own GPU (replicas: the path has no
 cross-volume exchange), so scaling is weak.
 """
@@ -217,9 +217,10 @@ def run_reference(args, rank):
     from qpop_diffraction_b200 import workloads
     diffraction = reference_diffraction()
     kind, cores = "reference", os.cpu_count()  # as the reference runs: NumPy's own threading
-    if diffraction is None:  # no install and no checkout: the oracle port, the same algorithm restated
-        from oracle import diffraction_oracle as oracle
-        diffraction, kind = oracle.diffraction, "port"
+    if diffraction is None:  # a restatement of ours would not be the reference
+        print(json.dumps({"impl": "reference", "unavailable": "the reference package is not installed (baseline/_ref) "
+                                                              "and no source checkout is present"}), flush=True)
+        return
     cases = [workloads.config2(shape=REF_SAMPLE, hkl=h) for h in REFLECTIONS]
     for i in range(args.warmup):
         diffraction(*cases[i % 2].args())
@@ -229,8 +230,7 @@ def run_reference(args, rank):
     dt = time.perf_counter() - t
     n = cases[0].params.n
     value = args.steps * n / dt / 1e9
-    who = "the reference's own diffraction() (baseline/_ref, unmodified, NumPy as installed)" if kind == "reference" else \
-          "the oracle port of the reference's diffraction() (NumPy)"
+    who = "the reference's own diffraction() (baseline/_ref, unmodified, NumPy as installed)"
     sample = (f"{who} on the config-2 snapshot cropped to {'x'.join(map(str, REF_SAMPLE))}, G=002,103 alternating, "
               f"one crop per step; host {host_cpu()}")
     print(json.dumps({
