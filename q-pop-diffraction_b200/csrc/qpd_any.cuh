@@ -8,11 +8,14 @@
 //
 // They are bound by instruction issue and by the latency of the stages' barriers (issue slots 55% busy, 13 warps
 // per SM at 128 registers; caps of 80 and 64 registers measured slower), not by memory: 91 instructions per
-// transformed value against 430 of the general kernels they replace.  One B200, float32, us before -> after:
-//   150x135x75    z stage 464 -> 159, y pass 715 -> 101, x pass 252 -> 41
-//   240x200x60    z stage 889 -> 348, y pass 919 -> 225, x pass 372 -> 72 (dense weights)
-//   1x400x400     z stage 87 -> 40, y pass 269 -> 33, x pass 39 -> 19
-//   120x100x50    adjoint: seed 112 -> 35, x and y passes 318 -> 87, z stage 244 -> 82
+// transformed value against 430 of the general kernels (150x135x75, whose lengths qpd_zcol.cuh and qpd_axisct.cuh take
+// now).  One B200, float32, us, general kernels (qpd_kernels.cuh) -> here, at sizes that these take:
+//   240x200x60 z stage, dense weights    889 -> 345
+//   1x400x400 z stage                    87 -> 40
+//   120x100x50 adjoint z stage           244 -> 82
+//   x pass of Nx64x32    1080: 300 -> 105, 1536: 354 -> 134, 2000: 431 -> 207, 3000: 637 -> 297, 4096: 816 -> 480,
+//                        6000: 1379 -> 959 (8192: 1801, on the general kernels: the tile exceeds 8192 values)
+//   y pass of 64xNx32    1080: 907 -> 240, 2000: 1263 -> 516, 3000: 1993 -> 762, 4096: 2316 -> 1275, 5000: 3044 -> 1749
 //
 // The pass over y or x (axis_any) walks its input fields with the next one's tile arriving by cp.async in a
 // second buffer while the current one is transformed; every thread owns one pencil and rows k0, k0 + K, ...
@@ -161,11 +164,9 @@ __global__ void __launch_bounds__(512) axis_any(const __grid_constant__ AxisAny<
         else cp_async_commit();
         const C* cf = static_cast<const C*>(g.f.coef[i]);
         C cfr[EPT];
-        if (cf) {
 #pragma unroll
-            for (int q = 0; q < EPT; q++)
-                if (q < rows) cfr[q] = __ldg(cf + k0 + q * K);
-        }
+        for (int q = 0; q < EPT; q++)
+            if (q < rows) cfr[q] = __ldg(cf + k0 + q * K);
         cp_async_wait<1>();
         if constexpr (MODE == AnyMode::Pre) {
 #pragma unroll
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(512) axis_any(const __grid_constant__ AxisAny<
         for (int q = 0; q < EPT; q++) {
             if (q < rows) {
                 const C v = res[q * nt];
-                if (MODE == AnyMode::Pre || !cf) acc[q] = cadd(acc[q], v);
+                if (MODE == AnyMode::Pre) acc[q] = cadd(acc[q], v);
                 else fold_fma(acc[q], cfr[q], v);
             }
         }
@@ -233,8 +234,7 @@ template <typename T, AnyMode MODE> __global__ void __launch_bounds__(256) axis_
     C acc = cmake<C>(0, 0);
     for (int i = 0; i < g.f.n; i++) {
         const C v = a.in[(long long)g.f.field[i] * a.fstride + base];
-        const C* cf = static_cast<const C*>(g.f.coef[i]);
-        fold_fma(acc, cf ? __ldg(cf) : cmake<C>(1, 0), v);
+        fold_fma(acc, __ldg(static_cast<const C*>(g.f.coef[i])), v);
         if (!g.f.last[i]) continue;
         C* dst = a.out + (long long)g.f.out[i] * a.fstride + base;
         if constexpr (MODE == AnyMode::Store || MODE == AnyMode::Pre) {

@@ -1,5 +1,5 @@
-// Runtime-length passes (qpd_any.cuh) behind the fused schedule, its adjoint and the plain schedule: any axis
-// whose length is a product of factors up to 17 and whose tile fits shared memory.
+// Runtime-length passes (qpd_any.cuh) behind the fused schedule and its adjoint: any axis whose length is a product
+// of factors up to 17 and whose tile fits shared memory.  (The plain schedule runs the general kernels.)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -8,7 +8,9 @@
 
 namespace qpd {
 
-constexpr int kAnyInputs = 64;  // inputs of one pass
+// Inputs of one pass: the size of the list that travels as a kernel parameter.  A crystal of more than 21 distinct
+// (R_x, R_y) has more in its y pass, which the kernels of qpd_fast.cuh and qpd_kernels.cuh run then.
+constexpr int kAnyInputs = 64;
 constexpr int kAnyStages = 8;
 
 // Stages of one axis, radices up to 17, and its twiddles on the device in the order the stages read them: for
@@ -26,8 +28,8 @@ __host__ __device__ constexpr int any_tw_row(int R) { return R / 2 * 2; }
 bool any_stages(long long N, AnyStages* p);
 void any_twiddles(const AnyStages& p, double2* tw);  // ntw values
 
-// The inputs of one pass in segment order: input i is field[i] times coef[i][k] (null: 1), and closes the
-// output out[i] when last[i].
+// The inputs of one pass in segment order: input i is field[i] times coef[i][k], and closes the output out[i]
+// when last[i]; n = 0: not a pass that these kernels take.
 struct AnyFold {
     int n = 0;
     short field[kAnyInputs];

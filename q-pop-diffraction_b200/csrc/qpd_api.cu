@@ -115,12 +115,13 @@ struct qpd_ctx {
     bool fast = true;
     // launch-shape choices among equivalent kernels: QPOP_B200_ZCFG=1 (z stage, nz = 104: 416 threads
     // reading inputs from shared memory instead of 256 holding them in registers),
-    // QPOP_B200_NBUF (tile buffers of the TMA passes, 2 or 3)
+    // QPOP_B200_NBUF (tile buffers of the TMA passes, 2 or 3).  A choice that is not the default also puts zcol
+    // (z stage) or axis_ct (y and x passes, float32) aside, whose place these kernels had.
     int knob_z = 0;
     int knob_nbuf = 2;
-    // z stage for nz = 104 and 68: the register-fused prime-factor kernel (zstage_pfa) or the Stockham one.
-    // Default (-1): fused for nz = 68 (69.8 against 89.3 ms at 4000x4000x68), Stockham for nz = 104 (1.81
-    // against 1.84 ms at 512x512x104); QPOP_B200_ZPFA=0 or 1 forces one of them for both lengths.
+    // z stage for nz = 104 and 68: QPOP_B200_ZPFA=1 the register-fused prime-factor kernel (zstage_pfa), 0 the
+    // Stockham one.  Default (-1): zcol for single-phase inputs; where it does not fit or is put aside, fused for
+    // nz = 68 (69.8 against 89.3 ms at 4000x4000x68, which keeps it) and Stockham for nz = 104 (1.81 against 1.84 ms).
     int knob_zpfa = -1;
     // QPOP_B200_N4000: launch shape of the 4000-point passes (0: 512 threads, out-of-place swizzled
     // stages; 1: one buffer, two CTAs per SM; 2: 1024 threads in place; 3: 512 threads in place;
@@ -130,7 +131,7 @@ struct qpd_ctx {
     // the z stage's fields with y fastest so the 4000-point y transforms read contiguous pencils)
     int knob_yfast = 1;
     int knob_bulk_nt = 256;
-    // QPOP_B200_ZREGIN=0: nz = 64 and 128 z stages with 512 threads reading their inputs from shared
+    // QPOP_B200_ZREGIN=0 (instead of zcol): nz = 64 and 128 z stages with 512 threads reading their inputs from shared
     // memory for every atom, instead of 256 threads holding them in registers (0.262 against 0.239 ms
     // at 256x256x64, 0.156 against 0.142 ms at 128^3)
     int knob_zregin = 1;
@@ -669,6 +670,10 @@ template <typename T> struct Impl {
             if (total > kAnyInputs) return;
             for (auto& s : segs)
                 for (int i = 0; i < s.nin; i++, f->n++) {
+                    if (!s.coef[0][i]) {  // the plain schedule's identity: not a fold
+                        f->n = 0;
+                        return;
+                    }
                     f->field[f->n] = (short)s.in[i];
                     f->out[f->n] = (short)s.out[0];
                     f->last[f->n] = i + 1 == s.nin;
@@ -766,18 +771,21 @@ template <typename T> struct Impl {
     }
 
     // y or x pass (axis d) on the compile-time register-folding kernels; nfields: fields of the buffer at a.in.
-    // They take every length that they have, 24 to 1024 (N x N x 32: 1.4 to 2.7 times faster than the runtime-length
-    // passes over the list, with odd nz 101 -> 69 for the y pass at 150x135x75; against axis_tma, us: y pass 1015 -> 745 and x pass
-    // 397 -> 306 at 512x512x104, 3870 -> 2285 and 1577 -> 961 at 1024x1024x68, 167 -> 110 and 74 -> 58 at 256x256x64,
-    // 86 -> 60 and 39 -> 31 at 128^3; the adjoint's x and y passes 395 -> 164 at 256x256x64).
+    // They take every length that they have, 24 to 1024, but odd nz only where ct_odd_nz says so.  N x N x 32: 1.4 to 2.7
+    // times faster than the runtime-length passes over the list.  Thin volumes fill a tile of 8 z values in part and
+    // still gain: N x N x nz with N from 25 to 1000 and nz from 1 to 17 are as fast or up to 2.8 times faster (300x300x8:
+    // y pass 98 -> 36, x pass 46 -> 19), except nz = 1 to 3 from 225 points on (300x300x1: 31 -> 42 and 17 -> 21;
+    // 1000x1000x2: 176 -> 201) and nz = 9 and 17 at 150 and 225 (27 -> 29, 35 -> 39).  Against axis_tma, us: y pass
+    // 1015 -> 745 and x pass 397 -> 306 at 512x512x104, 3870 -> 2285 and 1577 -> 961 at 1024x1024x68, 167 -> 110 and
+    // 74 -> 58 at 256x256x64, 86 -> 60 and 39 -> 31 at 128^3; the adjoint's x and y passes 395 -> 164 at 256x256x64.
     static int ct_axis(qpd_ctx* c, const AxisArgs<T>& a, int d, const AnyFold& f, AnyMode mode, int64_t nfields, int kind,
                        cudaStream_t st, bool* done) {
         *done = false;
         if constexpr (sizeof(T) == 4) {
             const AxisCtShape& s = c->ct[d];
             // a launch shape chosen for axis_tma keeps it
-            if (!c->fast || !c->tma || c->knob_oop != 1 || c->knob_nbuf != 2 || (kind >= QPD_K_ADJSEED && !c->knob_adj_tma) ||
-                s.cz == 0 || f.n == 0 || a.accumulate)
+            if (!c->fast || !c->tma || c->knob_oop != 1 || c->knob_nbuf != 2 ||
+                (kind >= QPD_K_ADJSEED && !c->knob_adj_tma) || s.cz == 0 || f.n == 0 || a.accumulate)
                 return QPD_OK;
             CUtensorMap map;
             const bool even = a.nz % 2 == 0;  // the map's row strides are multiples of 16 bytes
@@ -787,7 +795,8 @@ template <typename T> struct Impl {
                                   d == 0 ? 1 : s.box, d == 0 ? s.box : 1));
             cudaEvent_t t0;
             QPD_TRY(tstart(c, st, &t0));
-            QPD_CU(c, launch_axis_ct(even ? &map : nullptr, a, f, static_cast<const C*>(s.stages.tw), mode, d == 0, d == 0 ? c->ny : c->nx, st));
+            QPD_CU(c, launch_axis_ct(even ? &map : nullptr, a, f, static_cast<const C*>(s.stages.tw), mode, d == 0,
+                                     d == 0 ? c->ny : c->nx, st));
             *done = true;
             return tstop(c, kind, st, t0);
         }
@@ -795,10 +804,11 @@ template <typename T> struct Impl {
     }
 
     // y or x pass (axis d) on the runtime-length kernels; *done is false when they do not cover it.  They take the
-    // lengths without a compile-time kernel (measured against the general kernels, us: y pass 101 against 715 and x
-    // pass 41 against 252 at 150x135x75; against the compile-time ones they lose, 1940 to 1014 for the y pass at
-    // 512x512x104); what they do not cover, a prime factor above 17 or a tile beyond shared memory, stays on the
-    // general kernels.
+    // lengths without a compile-time kernel, from 1 to about 6000: 1.3 to 4 times faster than the general kernels from
+    // 1040 to 6000 points, where their tiles fall to 4, 2 and 1 pencils (us at both ends: x pass 268 -> 103 at 1040x64x32,
+    // 1379 -> 959 at 6000x64x32; figures in qpd_any.cuh); the compile-time ones beat them (y pass 1014 against 1940 at
+    // 512x512x104).  What they do not cover, a prime factor above 17, a tile beyond 8192 values or shared memory, or more
+    // than kAnyInputs inputs, stays on the general kernels.
     static int any_axis(qpd_ctx* c, const AxisArgs<T>& a, int d, const AnyFold& f, AnyMode mode, int kind,
                         cudaStream_t st, bool* done) {
         *done = false;
@@ -849,8 +859,9 @@ template <typename T> struct Impl {
         return tstop(c, QPD_K_ADJAXIS, st, t0);
     }
 
-    // adjoint x / y pass on the TMA kernel (coefficients before the transform), for the lengths the
-    // forward specialises; nfields_in: fields of the adjoint workspace the input lives in
+    // adjoint x / y pass of 256 or 512 points on the TMA kernel (coefficients before the transform); nfields_in: fields
+    // of the adjoint workspace the input lives in.  axis_ct takes these lengths (395 -> 164 us at 256x256x64): only
+    // QPOP_B200_OOP=0 and QPOP_B200_NBUF=3 lead here, and to the seed's TMA form in adjoint().
     template <int N, int NT, class RAD>
     static int adj_tma_(qpd_ctx* c, AxisArgs<T>& a, int64_t nouter, bool xp, cudaStream_t st, int64_t nfields_in) {
         if (xp) return tma_axis_b<N, 8, NT, 2, false, true, RAD, 2, true, false, true>(c, a, nouter, QPD_K_ADJAXIS, st,
@@ -1007,9 +1018,9 @@ template <typename T> struct Impl {
         constexpr bool F = sizeof(T) == 4;
         if constexpr (F) {
             // single-phase inputs of a covered nz (us, before -> after): 1826 -> 1530 at 512x512x104, 4457 -> 3980 at
-            // 1024x1024x68, 238 -> 187 at 256x256x64, 144 -> 116 at 128^3, and against the runtime-length z stage 159 -> 98
-            // at 150x135x75, 74 -> 48 at 120x100x50.  A z stage chosen by a switch keeps it, and
-            // both routes of the y-fastest grid keep the arithmetic of that route's z stage (zstage_pfa).
+            // 1024x1024x68, 238 -> 187 at 256x256x64, 144 -> 116 at 128^3, and against the runtime-length z stage
+            // 159 -> 98 at 150x135x75, 74 -> 48 at 120x100x50.  A z stage chosen by a switch keeps it, and both routes of
+            // the y-fastest grid keep the arithmetic of that route's z stage (zstage_pfa).
             if (c->knob_zpfa < 0 && c->knob_z == 0 && c->knob_zregin == 1 && !yfast_grid(c)) {
                 cudaEvent_t t0;
                 QPD_TRY(tstart(c, st, &t0));
@@ -1619,7 +1630,8 @@ template <typename T> struct Impl {
             return at.type == cudaMemoryTypeUnregistered;
         };
         const bool helped = c->workers->size() > 0;
-        const bool paged = helped && (pageable(oPhase) || pageable(u) || (NS > 0 && pageable(oStruc)) || (region && pageable(region)));
+        const bool paged = helped && (pageable(oPhase) || pageable(u) || (NS > 0 && pageable(oStruc)) ||
+                                      (region && pageable(region)));
         int64_t C = std::min<int64_t>(n, (int64_t)1 << 21);  // cells per chunk
         if (paged) C = std::min<int64_t>(C, std::max<int64_t>((int64_t)1 << 16, ((n + 3) / 4 + 63) / 64 * 64));
         constexpr int NSLOT = 3;
@@ -1711,10 +1723,11 @@ template <typename T> struct Impl {
                 });
                 const uint32_t f = fl.load();
                 flags |= f;
-                // the 3 planes of P and the 3 of U follow one another on both sides: one 2-D copy for the small chunks of
-                // pageable arrays (its pitch is at most 2^31 - 1 bytes), six plain ones for the large ones
+                // the 3 planes of P and the 3 of U follow one another on both sides: one 2-D copy for chunks of pageable
+                // arrays (its pitch is at most 2^31 - 1 bytes), else six plain ones
                 if (paged && sizeof(T) * (size_t)n <= (size_t)0x7fffffff) {
-                    QPD_CU(c, cudaMemcpy2DAsync(P + g0, sizeof(T) * n, h.P, sizeof(T) * C, sizeof(T) * cnt, 6, cudaMemcpyHostToDevice, st));
+                    QPD_CU(c, cudaMemcpy2DAsync(P + g0, sizeof(T) * n, h.P, sizeof(T) * C, sizeof(T) * cnt, 6,
+                                                cudaMemcpyHostToDevice, st));
                 } else {
                     for (int k = 0; k < 6; k++)
                         QPD_CU(c, cudaMemcpyAsync(P + k * n + g0, h.P + k * C, sizeof(T) * cnt, cudaMemcpyHostToDevice, st));
@@ -1763,11 +1776,13 @@ template <typename T> struct Impl {
         } else {
             // a pageable result comes through the pinned ring, piece by piece, the workers copying (and touching the
             // pages of) the pieces that have landed
-            const size_t piece = std::min((c->hring_bytes / NSLOT) & ~size_t(4095), std::max<size_t>(((total / 8) & ~size_t(4095)) + 4096, (size_t)1 << 18));
+            const size_t page = 4096, slot = c->hring_bytes / NSLOT / page * page;
+            const size_t piece = std::min(slot, std::max<size_t>(total / 8 / page * page + page, (size_t)1 << 18));
             const int64_t np = (int64_t)((total + piece - 1) / piece);
             auto fetch = [&](int64_t i) -> int {
                 const size_t at = i * piece, len = std::min(piece, total - at);
-                QPD_CU(c, cudaMemcpyAsync(static_cast<char*>(c->hring) + (i % NSLOT) * piece, reinterpret_cast<char*>(Id) + at, len, cudaMemcpyDeviceToHost, st));
+                QPD_CU(c, cudaMemcpyAsync(static_cast<char*>(c->hring) + (i % NSLOT) * piece,
+                                          reinterpret_cast<char*>(Id) + at, len, cudaMemcpyDeviceToHost, st));
                 QPD_CU(c, cudaEventRecord(c->ring_ev[i % NSLOT], st));
                 return QPD_OK;
             };
@@ -2127,7 +2142,6 @@ int qpd_pack_fields(qpd_ctx* c, const qpd_fields* in, void* P, void* U, int8_t* 
     for (int m = 0; m < in->n_material; m++)
         if (in->phase_of[m] < -1 || in->phase_of[m] >= c->nPhase)
             return fail(c, QPD_ERR_ARG, "qpd_pack_fields: phase_of[%d] = %d outside -1..%d", m, in->phase_of[m], c->nPhase - 1);
-    if (c->ny > 65535) return fail(c, QPD_ERR_UNSUPPORTED, "qpd_pack_fields: ny %lld > 65535", (long long)c->ny);
     if (in->z0 < 0 || in->z0 + c->nz > in->nz_full)
         return fail(c, QPD_ERR_ARG, "qpd_pack_fields: crop z0 %lld + nz %lld outside the %lld-layer stack",
                     (long long)in->z0, (long long)c->nz, (long long)in->nz_full);

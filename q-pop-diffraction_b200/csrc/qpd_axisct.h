@@ -26,14 +26,14 @@ __host__ __device__ constexpr bool ct_odd_nz(int N) { return N < 512 && (N & (N 
 // reads (cz = 0: not covered).
 struct AxisCtShape {
     int cz = 0, box = 0;
-    bool odd_nz = false;      // loads its tiles by threads too
-
+    bool odd_nz = false;  // loads its tiles by threads too
     AnyStages stages;
 };
 AxisCtShape axis_ct_shape(int64_t N);
 
 // y pass (xpass false, nouter = nx) or x pass (nouter = ny) over (x, y, z) fields; map: the field array in boxes of
-// (2 cz, box, 1) or (2 cz, 1, box), or null (odd nz) for tiles loaded by the threads; tw: the twiddle rows of axis_ct_shape(N).stages.
+// (2 cz, box, 1) or (2 cz, 1, box), or null (odd nz) for tiles loaded by the threads; tw: the twiddle rows of
+// axis_ct_shape(N).stages.
 cudaError_t launch_axis_ct(const CUtensorMap* map, const AxisArgs<float>& a, const AnyFold& f, const float2* tw,
                            AnyMode mode, bool xpass, long long nouter, cudaStream_t st);
 

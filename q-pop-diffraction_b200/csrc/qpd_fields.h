@@ -46,7 +46,8 @@ template <typename T> struct FieldsArgs {
 
 constexpr int kFT = 32;        // tile edge (x and z)
 constexpr int kFRows = 8;      // threadIdx.y extent
-constexpr int kFieldsBlocks = 12 * 148;  // blocks that fill the device: three rounds of four per SM (6 and 8 per SM: 128^3 49 -> 52 us)
+// blocks that fill the device: three rounds of four per SM (with 6 and 8 per SM 128^3 takes 52 us instead of 49)
+constexpr int kFieldsBlocks = 12 * 148;
 constexpr int kFPitch = kFT + 1;
 
 template <typename T> cudaError_t launch_fields(const FieldsArgs<T>& a, cudaStream_t st);

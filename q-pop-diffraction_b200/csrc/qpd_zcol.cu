@@ -57,8 +57,10 @@ cudaError_t launch_zcol(const ZArgs<float>& a, int cta_tiles, int sms, size_t sm
     *done = false;
     if (a.in.wdense || a.yfast) return cudaSuccess;
     switch (a.nz) {
-#define QPD_ZCOL_CASE(A, B) \
-    case A * B: return pick<A, B, zcol_columns(A, B), ZCol<A, B, zcol_columns(A, B)>::NT <= 128 ? 4 : 3>(a, cta_tiles, sms, smem_max, st, done);
+#define QPD_ZCOL_CASE(A, B)                                                                            \
+    case A * B:                                                                                        \
+        return pick<A, B, zcol_columns(A, B), ZCol<A, B, zcol_columns(A, B)>::NT <= 128 ? 4 : 3>(a, cta_tiles, sms, smem_max, \
+                                                                                                 st, done);
         QPD_ZCOL_LENGTHS(QPD_ZCOL_CASE)
 #undef QPD_ZCOL_CASE
     }

@@ -16,11 +16,12 @@
 //     cell instead of four components) and each lane transforms two of the four components whole;
 //   - cells that do not scatter have a record of zeros, so the sources have no branches;
 //   - with isotropic ionic shifts (su = k delta, ISO) the phase is one fma on qC.P and the shifts are three.
-// Without pairs (N1 = 4 .. 7) a thread holds the N1 cells of its b alone.  Four CTAs of four warps at up to 128 registers beat three of eight at 80, which spill (1.53 against 1.92 ms at
-// 512x512x104, 3.98 against 4.97 at 1024x1024x68).  Folding in phase B's registers and storing from there halves
-// the exchanges but not the wavefronts (1.59 and 4.67 ms).  One B200, us per z stage, before (qpd_fast.cuh, for nz = 68
-// qpd_zpfa.cuh) -> now: 512x512x104 1826 -> 1528, 1024x1024x68 4457 -> 3977, 256x256x64 238 -> 187, 128^3 144 -> 117,
-// 64x64x32 18 -> 15; against the runtime-length stage (qpd_any.cuh) 150x135x75 159 -> 98, 120x100x50 74 -> 48.
+// Without pairs (N1 = 4 .. 7) a thread holds the N1 cells of its b alone.  Four CTAs of four warps at up to 128
+// registers beat three of eight at 80, which spill (1.53 against 1.92 ms at 512x512x104, 3.98 against 4.97 at
+// 1024x1024x68).  Folding in phase B's registers and storing from there halves the exchanges but not the wavefronts
+// (1.59 and 4.67 ms).  One B200, us per z stage, before (qpd_fast.cuh, for nz = 68 qpd_zpfa.cuh) -> now: 512x512x104
+// 1826 -> 1528, 1024x1024x68 4457 -> 3977, 256x256x64 238 -> 187, 128^3 144 -> 117, 64x64x32 18 -> 15; against the
+// runtime-length stage (qpd_any.cuh) 150x135x75 159 -> 98, 120x100x50 74 -> 48.
 #pragma once
 
 #include "qpd_kernels.cuh"
@@ -257,7 +258,10 @@ __global__ void __launch_bounds__(ZCol<N1, N2, M>::NT, MINB) zcol(const __grid_c
                     for (int q = 0; q < 4; q++) {
                         C v[CA];
 #pragma unroll
-                        for (int j = 0; j < CA; j++) v[j] = q == 0 ? E[j] : make_float2(E[j].x * ua[(q + 2) % 3][j], E[j].y * ua[(q + 2) % 3][j]);
+                        for (int j = 0; j < CA; j++) {
+                            const float u = ua[(q + 2) % 3][j];
+                            v[j] = q == 0 ? E[j] : make_float2(E[j].x * u, E[j].y * u);
+                        }
                         Bfly<CA, C>::run(v);
                         if constexpr (!L::PFA) {
 #pragma unroll
@@ -284,7 +288,7 @@ __global__ void __launch_bounds__(ZCol<N1, N2, M>::NT, MINB) zcol(const __grid_c
                         g1_[j] = __shfl_xor_sync(0xffffffffu, g1_[j], 1);
                     }
                     // lane 1 holds its cells 4 places early: its outputs of odd k carry a factor -1, undone on the
-                    // way out (zcol_sign)
+                    // way out, in the fold
 #pragma unroll
                     for (int q = 0; q < 2; q++) {
                         C v[8];
