@@ -516,8 +516,8 @@ cudaError_t launch_axis_any(const AxisArgs<T>& a, const AnyFold& f, const AnySta
     auto smem = [&](int lp) { return sizeof(C) * ((size_t)3 * (st.N << lp) + st.ntw); };
     int lp = sizeof(T) == 4 ? 3 : 2;
     while ((st.N << lp) < 1024 && lp < 8 && (1LL << lp) < npen) lp++;
-    while (lp > 0 && ((st.N << lp) > 8192 || smem(lp) > smem_max)) lp--;
-    if ((st.N << lp) > 8192 || smem(lp) > smem_max) return cudaSuccess;
+    while (lp > 0 && ((st.N << lp) > kAnyTile || smem(lp) > smem_max)) lp--;
+    if ((st.N << lp) > kAnyTile || smem(lp) > smem_max) return cudaSuccess;
     const int least = sizeof(T) == 4 ? 2 : 1;
     while (lp > least && (npen >> lp) < 2LL * sms) lp--;
     const int elems = st.N << lp;

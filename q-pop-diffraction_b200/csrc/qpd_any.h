@@ -12,6 +12,8 @@ namespace qpd {
 // (R_x, R_y) has more in its y pass, which the kernels of qpd_fast.cuh and qpd_kernels.cuh run then.
 constexpr int kAnyInputs = 64;
 constexpr int kAnyStages = 8;
+// The longest axes that their tiles hold: one pencil of 8192 values (y and x), one column of 512 threads x 4 cells (z).
+constexpr int kAnyTile = 8192, kAnyColumn = 2048;
 
 // Stages of one axis, radices up to 17, and its twiddles on the device in the order the stages read them: for
 // each stage after the first and each k < Ns the row exp(-2 pi i r k / (Ns R)), r = 1 .. R - 1, padded to an

@@ -1809,7 +1809,7 @@ template <typename T> struct Impl {
 // passes and of the compile-time ones, each where a 16-byte load can start.
 int upload_twiddles(qpd_ctx* c, int d, int64_t N) {
     c->any[d] = AnyStages();
-    c->any_ok[d] = any_stages(N, &c->any[d]);
+    c->any_ok[d] = N <= (d == 2 ? kAnyColumn : kAnyTile) && any_stages(N, &c->any[d]);
     c->ct[d] = AxisCtShape();
     if (c->precision == QPD_FP32 && d < 2) c->ct[d] = axis_ct_shape(N);
     const size_t at_any = (N + 1) / 2 * 2, at_ct = at_any + (c->any_ok[d] ? c->any[d].ntw : 0);

@@ -133,3 +133,12 @@ def test_more_fold_inputs_than_a_pass_takes(gpu, monkeypatch, atoms):
     case.atoms.xAtom[:, 0] = np.arange(atoms) % 5 / 5 + 0.05  # five R_x, so that the fused schedule holds them
     for precision in ("fp32", "fp64"):
         against_general(gpu, monkeypatch, case, precision)
+
+
+@pytest.mark.parametrize("shape,n", [((16384, 1, 1), 16384), ((1, 9000, 1), 9000), ((1, 1, 4096), 4096)])
+def test_no_tables_for_lengths_beyond_the_tiles(gpu, shape, n):
+    """An axis longer than any tile of the runtime-length passes holds its N twiddles and no rows for those passes."""
+    from qpop_diffraction_b200 import Plan
+    with Plan(shape, (0.4, 0.4, 0.4), 1) as plan:
+        rest = 256 + 2 * 2 * 8  # the status word, and the tables of two axes of length 1
+        assert plan.workspace_bytes == 8 * n + rest
