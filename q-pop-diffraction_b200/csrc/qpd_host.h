@@ -15,6 +15,7 @@
 #include <functional>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -26,8 +27,13 @@ namespace qpd {
 // out of one job still holds that job, whose indices are used up, and cannot take or count an index of the next.
 class Workers {
    public:
+    // n threads, or as many of them as the system gives: the calling thread takes the rest of every job
     explicit Workers(int n) {
-        for (int i = 0; i < n; i++) th_.emplace_back([this] { loop(); });
+        th_.reserve(n > 0 ? n : 0);
+        try {
+            for (int i = 0; i < n; i++) th_.emplace_back([this] { loop(); });
+        } catch (const std::system_error&) {
+        }
     }
     ~Workers() {
         {
